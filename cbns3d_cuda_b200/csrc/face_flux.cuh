@@ -13,22 +13,44 @@
 // same use of the node primitives for the Roe average.  The algebra is
 // reorganised for the GPU (all of it is exact rearrangement, so results agree to
 // rounding):
-//   * the 6 stencil states are projected onto the characteristic fields once;
-//     the low-side stencil uses points 0..4 and the high-side stencil the same
-//     projected values 5..1, instead of projecting 10 states;
+//   * WENO5 in differences: a reconstructed value is the centre node's value
+//     plus a combination of the five first differences g1..g5 of the stencil,
+//     and the smoothness indicators are quadratic in the same differences.  The
+//     projection is linear, so the five differences of the conservative states
+//     are projected (not the six states, nor ten), and the projected-back
+//     correction is added to the centre node's conservative state, which is
+//     never projected.  The differences of neighbouring states carry less
+//     rounding than combinations of the states themselves;
+//   * the two sides share the four second differences of a field, whose squares
+//     enter three indicators each; the indicators are kept times 4 (and times
+//     the projection's scale squared), which the weights cancel;
 //   * the left eigenvectors are applied through their structure
 //     (w0,w2 = A +- B, w1 = f0 - 2A, w3,w4 = tangential momenta) and the right
-//     eigenvectors likewise, instead of 5x5 matrix products;
-//   * each WENO5 value costs one division (weights scaled by the product of
-//     the squared smoothness indicators); in FP64 the two sides of a field
-//     share it, and so do the two densities of the Roe average and of the
-//     reconstructed states (simultaneous inversion), and the second tangent
-//     is normalised with the product of the other two norms; the FP32 form
-//     uses fast reciprocals.
-// FP32 reciprocals and square roots are the approximate hardware forms (PTX
-// rcp.approx.ftz / sqrt.approx.ftz, within 2 ulp): the FP32 flux carries ~1e-7
-// relative error anyway, and the correctly rounded forms cost a Newton step and
-// a special-case branch each (11% of the hybrid stage kernel's time).
+//     eigenvectors likewise, instead of 5x5 matrix products; the second
+//     tangent is the cross product of the unit normal and the first;
+//   * each WENO5 value takes one reciprocal (weights scaled by the product of
+//     the squared indicators);
+//   * the Lax-Friedrichs flux is formed from the reconstructed conservative
+//     values, each side's collected into one coefficient ((q_n +- ws)/2).
+// About 690 FP64 instructions per face (projecting the states, with each side's
+// indicators and IEEE divisions and roots, took about 1,150).  Every operation
+// is an explicit fused multiply-add, multiply or add, so each compilation of
+// the flux (stage kernels, their batched forms, the WENO5-face pass) rounds
+// alike.  Bound by the FP64 pipe (FP64) and by issue (FP32).  Measured, one
+// launch each: FP64 stage 2 on 256x256x128 2.19 -> 1.86 ms, FP32 stage 2 on
+// 193x161x129 0.645 -> 0.480 ms, the WENO5-face pass of a 256x256x128 hybrid
+// step 0.208 -> 0.171 ms; the error of a right-hand side against 80-bit
+// arithmetic falls by 1.1 to 3 times (density and energy of a vortex 6.5e-15
+// and 7.7e-14 -> 3.9e-15 and 4.3e-14 in FP64, 2.9e-6 and 3.6e-5 -> 2.1e-6 and
+// 2.3e-5 with the FP32 flux).
+//
+// Reciprocals and square roots: FP32 uses the approximate hardware forms (PTX
+// rcp.approx.ftz / rsqrt.approx.ftz / sqrt.approx.ftz, within 2 ulp): the FP32
+// flux carries ~1e-7 relative error anyway.  FP64 starts from the hardware's
+// 20-bit approximations and takes one third-order Householder iteration
+// (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
+// 1970), three and five fused operations, which leaves at most 1 ulp where the
+// library's correctly rounded forms cost several times as much.
 // R is the arithmetic type (double for the plain path, float for the split path).
 #pragma once
 
@@ -41,139 +63,107 @@ struct FluxConsts {
   R gamma, gam1, gam1_inv;
 };
 
-template <typename R>
-__device__ __forceinline__ R rcp_(R x) {
-  if constexpr (sizeof(R) == 8) {
-    return 1.0 / x;
-  } else {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-  }
+// one rounding each, never contracted
+__device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double ml(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float ml(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float ad(float a, float b) { return __fadd_rn(a, b); }
+
+// 1/x.  FP64: r(1 + e + e^2) with e = 1 - x r, r the 20-bit approximation (error e^3 ~ 2^-60).
+__device__ __forceinline__ double rcp_(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fm(-x, r, 1.0);
+  return fm(r, fm(e, e, e), r);
+}
+__device__ __forceinline__ float rcp_(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// 1/sqrt(x).  FP64: y(1 + e/2 + 3e^2/8) with e = 1 - x y^2.
+__device__ __forceinline__ double rsqrt_(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fm(ml(-x, y), y, 1.0);
+  return fm(ml(y, e), fm(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ float rsqrt_(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// sqrt(x); FP64: x rsqrt(x), 0 at 0
+__device__ __forceinline__ double sqrt_(double x) { return x == 0.0 ? x : ml(x, rsqrt_(x)); }
+__device__ __forceinline__ float sqrt_(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
+// Scale of the differences WENO5 works on: the indicators' fourth powers stay
+// inside FP32 for differences up to 7e5 (eps enters at 4e-9); FP64 takes the
+// 1/6 of the candidate values here.
 template <typename R>
-__device__ __forceinline__ R sqrt_(R x) {
-  if constexpr (sizeof(R) == 8) {
-    return sqrt(x);
-  } else {
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-  }
-}
+struct WenoScale {
+  static constexpr R s = sizeof(R) == 8 ? R(1.0 / 6.0) : R(1.0 / 32.0);  // of the projected differences
+  static constexpr R post = sizeof(R) == 8 ? R(1) : R(32.0 / 6.0);       // of the correction
+};
 
+// WENO5-JS of one field from its differences g1..g5 (scaled): the correction
+// to the centre value of the low side (stencil points 0..4, centre 2) and of
+// the high side (points 5..1, centre 3), before WenoScale::post.  eps4 = 4 eps
+// scale^2.
 template <typename R>
-__device__ __forceinline__ R div_(R a, R b) {
-  if constexpr (sizeof(R) == 8) {
-    return a / b;
-  } else {
-    return __fdividef(a, b);
-  }
-}
-
-// WENO5-JS value at the +1/2 side of c from the stencil a b c d e.
-template <typename R>
-__device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
-  const R eps = R(1.0e-6);
-  const R c13 = R(13.0 / 12.0);
-  const R d1 = a - R(2) * b + c, e1 = a - R(4) * b + R(3) * c;
-  const R d2 = b - R(2) * c + d, e2 = b - d;
-  const R d3 = c - R(2) * d + e, e3 = R(3) * c - R(4) * d + e;
-  const R s1 = c13 * d1 * d1 + R(0.25) * e1 * e1 + eps;
-  const R s2 = c13 * d2 * d2 + R(0.25) * e2 * e2 + eps;
-  const R s3 = c13 * d3 * d3 + R(0.25) * e3 * e3 + eps;
-  const R p1 = R(2) * a - R(7) * b + R(11) * c;  // 6 x candidate values
-  const R p2 = -b + R(5) * c + R(2) * d;
-  const R p3 = R(2) * c + R(5) * d - e;
-  if constexpr (sizeof(R) == 8) {
-    const R t1 = s1 * s1, t2 = s2 * s2, t3 = s3 * s3;
-    const R a1 = R(0.1) * (t2 * t3), a2 = R(0.6) * (t1 * t3), a3 = R(0.3) * (t1 * t2);
-    return (a1 * p1 + a2 * p2 + a3 * p3) / (R(6) * (a1 + a2 + a3));
-  } else {
-    const R a1 = __fdividef(R(0.1), s1 * s1);
-    const R a2 = __fdividef(R(0.6), s2 * s2);
-    const R a3 = __fdividef(R(0.3), s3 * s3);
-    return __fdividef(a1 * p1 + a2 * p2 + a3 * p3, R(6) * (a1 + a2 + a3));
-  }
-}
-
-// FP64 WENO5-JS values of the two sides of one characteristic field at once,
-// sharing one division: with the low side's value n_l/d_l and the high
-// side's n_h/d_h (weno5's numerator and denominator), 1/(d_l d_h) times d_h
-// and d_l gives both (simultaneous inversion, Montgomery 1987).  The
-// denominators are 6 (a1 + a2 + a3) with a_k ~ 1/s_k^2 scaled by s1^2 s2^2
-// s3^2, s_k >= 1e-6, so their product stays far inside the FP64 range.
-__device__ __forceinline__ void weno5_pair(double a, double b, double c, double d, double e, double f,
-                                           double* lo, double* hi) {
-  // low side from a b c d e, high side from f e d c b
-  auto nd = [](double a, double b, double c, double d, double e, double* n, double* den) {
-    const double eps = 1.0e-6, c13 = 13.0 / 12.0;
-    const double d1 = a - 2.0 * b + c, e1 = a - 4.0 * b + 3.0 * c;
-    const double d2 = b - 2.0 * c + d, e2 = b - d;
-    const double d3 = c - 2.0 * d + e, e3 = 3.0 * c - 4.0 * d + e;
-    const double s1 = c13 * d1 * d1 + 0.25 * e1 * e1 + eps;
-    const double s2 = c13 * d2 * d2 + 0.25 * e2 * e2 + eps;
-    const double s3 = c13 * d3 * d3 + 0.25 * e3 * e3 + eps;
-    const double p1 = 2.0 * a - 7.0 * b + 11.0 * c, p2 = -b + 5.0 * c + 2.0 * d, p3 = 2.0 * c + 5.0 * d - e;
-    const double t1 = s1 * s1, t2 = s2 * s2, t3 = s3 * s3;
-    const double a1 = 0.1 * (t2 * t3), a2 = 0.6 * (t1 * t3), a3 = 0.3 * (t1 * t2);
-    *n = a1 * p1 + a2 * p2 + a3 * p3;
-    *den = 6.0 * (a1 + a2 + a3);
+__device__ __forceinline__ void weno5_pair(R g1, R g2, R g3, R g4, R g5, R eps4, R* lo, R* hi) {
+  const R c = R(13.0 / 3.0);
+  const R d1 = ad(g2, -g1), d2 = ad(g3, -g2), d3 = ad(g4, -g3), d4 = ad(g5, -g4);
+  const R t2 = fm(ml(c, d2), d2, eps4), t3 = fm(ml(c, d3), d3, eps4);
+  auto side = [](R e1, R e2, R e3, R t1, R t2, R t3, R gn, R gc, R* out) {
+    // gn, gc: the difference next to the far pair and the one across the face
+    const R s1 = fm(e1, e1, t1), s2 = fm(e2, e2, t2), s3 = fm(e3, e3, t3);
+    const R p1 = ml(s2, s3), p2 = ml(s1, s3), p3 = ml(s1, s2);
+    const R u1 = ml(p1, p1), u2 = ml(R(6), ml(p2, p2)), u3 = ml(R(3), ml(p3, p3));
+    const R q1 = fm(R(2), e1, -gn), q2 = ad(e2, gc), q3 = ad(e3, gc);
+    const R n = fm(u3, q3, fm(u2, q2, ml(u1, q1)));
+    *out = ml(n, rcp_(ad(u3, ad(u2, u1))));
   };
-  double nl, dl, nh, dh;
-  nd(a, b, c, d, e, &nl, &dl);
-  nd(f, e, d, c, b, &nh, &dh);
-  const double r = 1.0 / (dl * dh);
-  *lo = nl * (dh * r);
-  *hi = nh * (dl * r);
+  const R t1 = fm(ml(c, d1), d1, eps4), t4 = fm(ml(c, d4), d4, eps4);
+  R h;
+  side(fm(R(2), g2, d1), ad(g2, g3), fm(R(2), g3, -d3), t1, t2, t3, g2, g3, lo);
+  side(fm(R(2), g4, -d4), ad(g3, g4), fm(R(2), g3, d2), t4, t3, t2, g4, g3, &h);
+  *hi = -h;
 }
 
-// Local Lax-Friedrichs flux from the two reconstructed states (the reference's
-// lf_flux with R = the high side H, L = the low side): the component-wise
-// Cartesian wave-speed bound, flux = (F_L + F_H - ws (U_H - U_L)) / 2.
+// Local Lax-Friedrichs flux from the two reconstructed conservative states
+// (the reference's lf_flux with R = the high side H, L = the low side): the
+// component-wise Cartesian wave-speed bound, flux = (F_L + F_H - ws (U_H -
+// U_L)) / 2.
 template <typename R>
-__device__ __forceinline__ void lf_flux_prims(R Lr, R Lu, R Lv, R Lw, R Lp, R Hr, R Hu, R Hv, R Hw, R Hp, R nx,
-                                              R ny, R nz, const FluxConsts<R>& C, R out[5]) {
-  const R gamma = C.gamma, gam1_inv = C.gam1_inv;
-  const R kH = Hu * Hu + Hv * Hv + Hw * Hw, kL = Lu * Lu + Lv * Lv + Lw * Lw;
-  const R cH = sqrt_(gamma * Hp * rcp_(Hr)), cL = sqrt_(gamma * Lp * rcp_(Lr));
-  const R HH = cH * cH * gam1_inv + R(0.5) * kH, HL = cL * cL * gam1_inv + R(0.5) * kL;
-  const R EH = Hp * gam1_inv + R(0.5) * Hr * kH, EL = Lp * gam1_inv + R(0.5) * Lr * kL;
-  const R qH = Hu * nx + Hv * ny + Hw * nz, qL = Lu * nx + Lv * ny + Lw * nz;
-  const R sx = fmax(fabs(Hu) + cH, fabs(Lu) + cL);
-  const R sy = fmax(fabs(Hv) + cH, fabs(Lv) + cL);
-  const R sz = fmax(fabs(Hw) + cH, fabs(Lw) + cL);
-  const R ws = fabs(sx * nx + sy * ny + sz * nz);
-  const R mL = Lr * qL, mH = Hr * qH;
-  out[0] = R(0.5) * (mL + mH - ws * (Hr - Lr));
-  out[1] = R(0.5) * (mL * Lu + Lp * nx + mH * Hu + Hp * nx - ws * (Hr * Hu - Lr * Lu));
-  out[2] = R(0.5) * (mL * Lv + Lp * ny + mH * Hv + Hp * ny - ws * (Hr * Hv - Lr * Lv));
-  out[3] = R(0.5) * (mL * Lw + Lp * nz + mH * Hw + Hp * nz - ws * (Hr * Hw - Lr * Lw));
-  out[4] = R(0.5) * (mL * HL + mH * HH - ws * (EH - EL));
-}
-
-// The same with the densities' reciprocals given (the FP64 face flux forms
-// them together).
-template <typename R>
-__device__ __forceinline__ void lf_flux_prims_inv(R Lr, R Lu, R Lv, R Lw, R Lp, R Hr, R Hu, R Hv, R Hw, R Hp, R iLr, R iHr, R nx,
-                                              R ny, R nz, const FluxConsts<R>& C, R out[5]) {
-  const R gamma = C.gamma, gam1_inv = C.gam1_inv;
-  const R kH = Hu * Hu + Hv * Hv + Hw * Hw, kL = Lu * Lu + Lv * Lv + Lw * Lw;
-  const R cH = sqrt_(gamma * Hp * iHr), cL = sqrt_(gamma * Lp * iLr);
-  const R HH = cH * cH * gam1_inv + R(0.5) * kH, HL = cL * cL * gam1_inv + R(0.5) * kL;
-  const R EH = Hp * gam1_inv + R(0.5) * Hr * kH, EL = Lp * gam1_inv + R(0.5) * Lr * kL;
-  const R qH = Hu * nx + Hv * ny + Hw * nz, qL = Lu * nx + Lv * ny + Lw * nz;
-  const R sx = fmax(fabs(Hu) + cH, fabs(Lu) + cL);
-  const R sy = fmax(fabs(Hv) + cH, fabs(Lv) + cL);
-  const R sz = fmax(fabs(Hw) + cH, fabs(Lw) + cL);
-  const R ws = fabs(sx * nx + sy * ny + sz * nz);
-  const R mL = Lr * qL, mH = Hr * qH;
-  out[0] = R(0.5) * (mL + mH - ws * (Hr - Lr));
-  out[1] = R(0.5) * (mL * Lu + Lp * nx + mH * Hu + Hp * nx - ws * (Hr * Hu - Lr * Lu));
-  out[2] = R(0.5) * (mL * Lv + Lp * ny + mH * Hv + Hp * ny - ws * (Hr * Hv - Lr * Lv));
-  out[3] = R(0.5) * (mL * Lw + Lp * nz + mH * Hw + Hp * nz - ws * (Hr * Hw - Lr * Lw));
-  out[4] = R(0.5) * (mL * HL + mH * HH - ws * (EH - EL));
+__device__ __forceinline__ void lf_flux(const R L[5], const R H[5], R nx, R ny, R nz, const FluxConsts<R>& C,
+                                        R out[5]) {
+  R pL, hL, sLx, sLy, sLz, pH, hH, sHx, sHy, sHz;  // pressure, q_n / 2, |u_i| + c
+  auto side = [&](const R q[5], R& p, R& h, R& sx, R& sy, R& sz) {
+    const R i = rcp_(q[0]);
+    const R u = ml(q[1], i), v = ml(q[2], i), w = ml(q[3], i);
+    p = ml(C.gam1, fm(R(-0.5), fm(q[3], w, fm(q[2], v, ml(q[1], u))), q[4]));
+    const R c = sqrt_(ml(ml(C.gamma, p), i));
+    h = ml(R(0.5), fm(w, nz, fm(v, ny, ml(u, nx))));
+    sx = ad(fabs(u), c);
+    sy = ad(fabs(v), c);
+    sz = ad(fabs(w), c);
+  };
+  side(L, pL, hL, sLx, sLy, sLz);
+  side(H, pH, hH, sHx, sHy, sHz);
+  const R ws = ml(R(0.5), fabs(fm(fmax(sHz, sLz), nz, fm(fmax(sHy, sLy), ny, ml(fmax(sHx, sLx), nx)))));
+  const R a = ad(hL, ws), b = ad(hH, -ws), hp = ml(R(0.5), ad(pL, pH));
+  out[0] = fm(H[0], b, ml(L[0], a));
+  out[1] = fm(hp, nx, fm(H[1], b, ml(L[1], a)));
+  out[2] = fm(hp, ny, fm(H[2], b, ml(L[2], a)));
+  out[3] = fm(hp, nz, fm(H[3], b, ml(L[3], a)));
+  out[4] = fm(pH, hH, fm(pL, hL, fm(H[4], b, ml(L[4], a))));
 }
 
 // Flux through the face between stencil points 2 (node a) and 3 (node b).
@@ -183,205 +173,131 @@ __device__ __forceinline__ void lf_flux_prims_inv(R Lr, R Lu, R Lv, R Lw, R Lp, 
 template <typename R, typename LD>
 __device__ __forceinline__ void face_flux(const LD& ld, R nx, R ny, R nz, const FluxConsts<R>& C,
                                           R out[5]) {
-  const R gamma = C.gamma, gam1 = C.gam1, gam1_inv = C.gam1_inv;
-
-  // node primitives at a and b (the reference reads them from the primitive
-  // arrays, which hold exactly these values on every node a face touches)
-  R ra, ua, va, wa, pa, rb, ub, vb, wb, pb, ira, irb;
-  if constexpr (sizeof(R) == 8) {
-    // both densities' reciprocals from one division
-    ra = ld(2, 0);
-    rb = ld(3, 0);
-    const R rab = rcp_(ra * rb);
-    ira = rb * rab;
-    irb = ra * rab;
-    ua = ld(2, 1) * ira;
-    va = ld(2, 2) * ira;
-    wa = ld(2, 3) * ira;
-    pa = gam1 * (ld(2, 4) - R(0.5) * ra * (ua * ua + va * va + wa * wa));
-    ub = ld(3, 1) * irb;
-    vb = ld(3, 2) * irb;
-    wb = ld(3, 3) * irb;
-    pb = gam1 * (ld(3, 4) - R(0.5) * rb * (ub * ub + vb * vb + wb * wb));
-  } else {
-    ra = ld(2, 0);
-    ira = rcp_(ra);
-    ua = ld(2, 1) * ira;
-    va = ld(2, 2) * ira;
-    wa = ld(2, 3) * ira;
-    pa = gam1 * (ld(2, 4) - R(0.5) * ra * (ua * ua + va * va + wa * wa));
-    rb = ld(3, 0);
-    irb = rcp_(rb);
-    ub = ld(3, 1) * irb;
-    vb = ld(3, 2) * irb;
-    wb = ld(3, 3) * irb;
-    pb = gam1 * (ld(3, 4) - R(0.5) * rb * (ub * ub + vb * vb + wb * wb));
-  }
-
-  // orthonormal basis (n, l, m)
-  R lx = R(0), ly = nz, lz = -ny, mx, my, mz;
-  if (ly * ly + lz * lz > R(1.0e-16)) {
-    mx = -ny * ny - nz * nz;
-    my = nx * ny;
-    mz = nx * nz;
-  } else {
-    lx = -nz;
-    ly = R(0);
-    lz = nx;
-    mx = nx * ny;
-    my = -nx * nx - nz * nz;
-    mz = ny * nz;
-  }
-  R ux, uy, uz;  // unit normal
+  // orthonormal basis (n, l, m): u, l, m = u x l
+  R ux, uy, uz, lx, ly, lz;
   {
-    const R in = rsqrt(nx * nx + ny * ny + nz * nz);
-    ux = nx * in;
-    uy = ny * in;
-    uz = nz * in;
-    const R il = rsqrt(lx * lx + ly * ly + lz * lz);
-    lx *= il;
-    ly *= il;
-    lz *= il;
-    // |m| = |l| |n| in both branches above (m = n x l up to sign)
-    R im;
-    if constexpr (sizeof(R) == 8) im = il * in;
-    else im = rsqrt(mx * mx + my * my + mz * mz);
-    mx *= im;
-    my *= im;
-    mz *= im;
-  }
-
-  // Roe averages
-  R uu, vv, ww, H, q2, c, qn, ql, qm, K, h;
-  {
-    const R Ha = gamma * pa * ira * gam1_inv + R(0.5) * (ua * ua + va * va + wa * wa);
-    const R Hb = gamma * pb * irb * gam1_inv + R(0.5) * (ub * ub + vb * vb + wb * wb);
-    const R sr = sqrt_(rb * ira);
-    const R is = rcp_(R(1) + sr);
-    uu = (ua + sr * ub) * is;
-    vv = (va + sr * vb) * is;
-    ww = (wa + sr * wb) * is;
-    H = (Ha + sr * Hb) * is;
-    q2 = uu * uu + vv * vv + ww * ww;
-    c = sqrt_(gam1 * (H - R(0.5) * q2));
-    const R ic = rcp_(c);
-    qn = uu * ux + vv * uy + ww * uz;
-    ql = uu * lx + vv * ly + ww * lz;
-    qm = uu * mx + vv * my + ww * mz;
-    h = R(0.5) * ic;
-    K = gam1 * h * ic;  // (gamma-1)/(2 c^2)
-  }
-
-  // characteristic projection of the 6 stencil states and WENO5 per field
-  // (low side from points 0..4, high side from 5..1).  FP64 projects all five
-  // fields in one pass; FP32 in two (acoustic + entropy fields, which share A
-  // and B, then the shear fields), which keeps at most 18 projected values live.
-  R wl[5], wh[5];
-  if constexpr (sizeof(R) == 8) {
-    R W[5][6];
-#pragma unroll
-    for (int p = 0; p < 6; ++p) {
-      const R f0 = ld(p, 0), f1 = ld(p, 1), f2 = ld(p, 2), f3 = ld(p, 3), f4 = ld(p, 4);
-      const R A = K * (R(0.5) * q2 * f0 - (uu * f1 + vv * f2 + ww * f3) + f4);
-      const R B = h * (qn * f0 - (ux * f1 + uy * f2 + uz * f3));
-      W[0][p] = A + B;
-      W[1][p] = f0 - R(2) * A;
-      W[2][p] = A - B;
-      W[3][p] = lx * f1 + ly * f2 + lz * f3 - ql * f0;
-      W[4][p] = mx * f1 + my * f2 + mz * f3 - qm * f0;
-    }
-#pragma unroll
-    for (int s = 0; s < 5; ++s) weno5_pair(W[s][0], W[s][1], W[s][2], W[s][3], W[s][4], W[s][5], &wl[s], &wh[s]);
-  } else {
-    {
-      R W[3][6];
-#pragma unroll
-      for (int p = 0; p < 6; ++p) {
-        const R f0 = ld(p, 0), f1 = ld(p, 1), f2 = ld(p, 2), f3 = ld(p, 3), f4 = ld(p, 4);
-        const R A = K * (R(0.5) * q2 * f0 - (uu * f1 + vv * f2 + ww * f3) + f4);
-        const R B = h * (qn * f0 - (ux * f1 + uy * f2 + uz * f3));
-        W[0][p] = A + B;
-        W[1][p] = f0 - R(2) * A;
-        W[2][p] = A - B;
-      }
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        wl[s] = weno5<R>(W[s][0], W[s][1], W[s][2], W[s][3], W[s][4]);
-        wh[s] = weno5<R>(W[s][5], W[s][4], W[s][3], W[s][2], W[s][1]);
-      }
-    }
-    {
-      R W[2][6];
-#pragma unroll
-      for (int p = 0; p < 6; ++p) {
-        const R f0 = ld(p, 0), f1 = ld(p, 1), f2 = ld(p, 2), f3 = ld(p, 3);
-        W[0][p] = lx * f1 + ly * f2 + lz * f3 - ql * f0;
-        W[1][p] = mx * f1 + my * f2 + mz * f3 - qm * f0;
-      }
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        wl[3 + s] = weno5<R>(W[s][0], W[s][1], W[s][2], W[s][3], W[s][4]);
-        wh[3 + s] = weno5<R>(W[s][5], W[s][4], W[s][3], W[s][2], W[s][1]);
-      }
-    }
-  }
-
-  // back to conservative variables, then primitives, on each side
-  R Lr, Lu, Lv, Lw, Lp, Hr, Hu, Hv, Hw, Hp;
-  {
-    const R hq = R(0.5) * q2;
-    R q[5];
-    auto back = [&](const R* w) {
-      const R s = w[0] + w[2], d = (w[2] - w[0]) * c;
-      q[0] = s + w[1];
-      q[1] = uu * q[0] + ux * d + lx * w[3] + mx * w[4];
-      q[2] = vv * q[0] + uy * d + ly * w[3] + my * w[4];
-      q[3] = ww * q[0] + uz * d + lz * w[3] + mz * w[4];
-      q[4] = H * s + qn * d + hq * w[1] + ql * w[3] + qm * w[4];
-    };
-    if constexpr (sizeof(R) == 8) {
-      // both sides' densities inverted with one division
-      back(wl);
-      R lq[5];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) lq[n] = q[n];
-      back(wh);
-      Lr = lq[0];
-      Hr = q[0];
-      const R rlh = rcp_(Lr * Hr), iL = Hr * rlh, iH = Lr * rlh;
-      Lu = lq[1] * iL;
-      Lv = lq[2] * iL;
-      Lw = lq[3] * iL;
-      Lp = gam1 * (lq[4] - R(0.5) * Lr * (Lu * Lu + Lv * Lv + Lw * Lw));
-      Hu = q[1] * iH;
-      Hv = q[2] * iH;
-      Hw = q[3] * iH;
-      Hp = gam1 * (q[4] - R(0.5) * Hr * (Hu * Hu + Hv * Hv + Hw * Hw));
-      lf_flux_prims_inv<R>(Lr, Lu, Lv, Lw, Lp, Hr, Hu, Hv, Hw, Hp, iL, iH, nx, ny, nz, C, out);
-      return;
+    const R yz = fm(nz, nz, ml(ny, ny));
+    const R in = rsqrt_(fm(nx, nx, yz));
+    ux = ml(nx, in);
+    uy = ml(ny, in);
+    uz = ml(nz, in);
+    if (yz > R(1.0e-16)) {
+      const R il = rsqrt_(yz);
+      lx = R(0);
+      ly = ml(nz, il);
+      lz = ml(-ny, il);
     } else {
-      back(wl);
-      Lr = q[0];
-      {
-        const R i = rcp_(Lr);
-        Lu = q[1] * i;
-        Lv = q[2] * i;
-        Lw = q[3] * i;
-        Lp = gam1 * (q[4] - R(0.5) * Lr * (Lu * Lu + Lv * Lv + Lw * Lw));
+      const R il = rsqrt_(fm(nz, nz, ml(nx, nx)));
+      lx = ml(-nz, il);
+      ly = R(0);
+      lz = ml(nx, il);
+    }
+  }
+  const R mx = fm(uy, lz, -ml(uz, ly)), my = fm(uz, lx, -ml(ux, lz)), mz = fm(ux, ly, -ml(uy, lx));
+
+  // Roe averages of the node primitives at a and b (the reference reads them
+  // from the primitive arrays, which hold exactly these values on every node a
+  // face touches)
+  R uu, vv, ww, H, hq, c, ic, qn, ql, qm;
+  {
+    auto node = [&](int p, R& i, R& u, R& v, R& w, R& h) {
+      i = rcp_(ld(p, 0));
+      u = ml(ld(p, 1), i);
+      v = ml(ld(p, 2), i);
+      w = ml(ld(p, 3), i);
+      const R E = ld(p, 4), k = fm(ld(p, 3), w, fm(ld(p, 2), v, ml(ld(p, 1), u)));
+      h = ml(fm(C.gam1, fm(R(-0.5), k, E), E), i);
+    };
+    R ia, ua, va, wa, Ha, ib, ub, vb, wb, Hb;
+    node(2, ia, ua, va, wa, Ha);
+    node(3, ib, ub, vb, wb, Hb);
+    const R sr = sqrt_(ml(ld(3, 0), ia));
+    const R is = rcp_(ad(R(1), sr));
+    uu = ml(fm(sr, ub, ua), is);
+    vv = ml(fm(sr, vb, va), is);
+    ww = ml(fm(sr, wb, wa), is);
+    H = ml(fm(sr, Hb, Ha), is);
+    hq = ml(R(0.5), fm(ww, ww, fm(vv, vv, ml(uu, uu))));
+    const R c2 = ml(C.gam1, ad(H, -hq));
+    ic = rsqrt_(c2);
+    c = ml(c2, ic);
+    qn = fm(ww, uz, fm(vv, uy, ml(uu, ux)));
+    ql = fm(ww, lz, fm(vv, ly, ml(uu, lx)));
+    qm = fm(ww, mz, fm(vv, my, ml(uu, mx)));
+  }
+
+  // characteristic projection of the five differences and WENO5 per field, in
+  // two groups (acoustic and entropy fields, which share A and B; shear
+  // fields), which keeps at most 15 projected values live
+  constexpr R S = WenoScale<R>::s;
+  R wl[5], wh[5];
+  {
+    R W[3][5];
+    {
+      const R K = ml(ml(S, C.gam1), ml(ic, ic));  // 2 S (gamma-1)/(2 c^2)
+      const R a0 = ml(K, hq), a1 = ml(-K, uu), a2 = ml(-K, vv), a3 = ml(-K, ww);
+      const R h = ml(R(0.5) * S, ic);
+      const R b0 = ml(h, qn), b1 = ml(-h, ux), b2 = ml(-h, uy), b3 = ml(-h, uz);
+#pragma unroll
+      for (int p = 0; p < 5; ++p) {
+        const R g0 = ad(ld(p + 1, 0), -ld(p, 0)), g1 = ad(ld(p + 1, 1), -ld(p, 1)), g2 = ad(ld(p + 1, 2), -ld(p, 2)),
+                g3 = ad(ld(p + 1, 3), -ld(p, 3)), g4 = ad(ld(p + 1, 4), -ld(p, 4));
+        const R A = fm(a3, g3, fm(a2, g2, fm(a1, g1, fm(a0, g0, ml(K, g4)))));  // 2 A
+        const R B = fm(b3, g3, fm(b2, g2, fm(b1, g1, ml(b0, g0))));
+        W[0][p] = fm(R(0.5), A, B);
+        W[1][p] = fm(S, g0, -A);
+        W[2][p] = fm(R(0.5), A, -B);
       }
-      back(wh);
-      Hr = q[0];
-      {
-        const R i = rcp_(Hr);
-        Hu = q[1] * i;
-        Hv = q[2] * i;
-        Hw = q[3] * i;
-        Hp = gam1 * (q[4] - R(0.5) * Hr * (Hu * Hu + Hv * Hv + Hw * Hw));
-      }
+    }
+#pragma unroll
+    for (int s = 0; s < 3; ++s)
+      weno5_pair(W[s][0], W[s][1], W[s][2], W[s][3], W[s][4], R(4.0e-6 * (double)S * (double)S), &wl[s], &wh[s]);
+  }
+  {
+    // FP64: unscaled here, the corrections scaled (4 products instead of 8)
+    constexpr R T = sizeof(R) == 8 ? R(1) : S;
+    R W[2][5];
+    const R l1 = ml(T, lx), l2 = ml(T, ly), l3 = ml(T, lz), l0 = ml(-T, ql);
+    const R m1 = ml(T, mx), m2 = ml(T, my), m3 = ml(T, mz), m0 = ml(-T, qm);
+#pragma unroll
+    for (int p = 0; p < 5; ++p) {
+      const R g0 = ad(ld(p + 1, 0), -ld(p, 0)), g1 = ad(ld(p + 1, 1), -ld(p, 1)), g2 = ad(ld(p + 1, 2), -ld(p, 2)),
+              g3 = ad(ld(p + 1, 3), -ld(p, 3));
+      W[0][p] = fm(l3, g3, fm(l2, g2, fm(l1, g1, ml(l0, g0))));
+      W[1][p] = fm(m3, g3, fm(m2, g2, fm(m1, g1, ml(m0, g0))));
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      weno5_pair(W[s][0], W[s][1], W[s][2], W[s][3], W[s][4], R(4.0e-6 * (double)T * (double)T), &wl[3 + s],
+                 &wh[3 + s]);
+  }
+  if constexpr (sizeof(R) == 8) {
+#pragma unroll
+    for (int s = 3; s < 5; ++s) {
+      wl[s] = ml(S, wl[s]);
+      wh[s] = ml(S, wh[s]);
+    }
+  } else {
+#pragma unroll
+    for (int s = 0; s < 5; ++s) {
+      wl[s] = ml(WenoScale<R>::post, wl[s]);
+      wh[s] = ml(WenoScale<R>::post, wh[s]);
     }
   }
 
-  lf_flux_prims<R>(Lr, Lu, Lv, Lw, Lp, Hr, Hu, Hv, Hw, Hp, nx, ny, nz, C, out);
+  // the corrections back to conservative variables, added to the centre nodes
+  R L[5], Hs[5];
+  auto back = [&](int p, const R* w, R* q) {
+    const R s = ad(w[0], w[2]), d = ml(ad(w[2], -w[0]), c), r = ad(s, w[1]);
+    q[0] = ad(ld(p, 0), r);
+    q[1] = fm(mx, w[4], fm(lx, w[3], fm(ux, d, fm(uu, r, ld(p, 1)))));
+    q[2] = fm(my, w[4], fm(ly, w[3], fm(uy, d, fm(vv, r, ld(p, 2)))));
+    q[3] = fm(mz, w[4], fm(lz, w[3], fm(uz, d, fm(ww, r, ld(p, 3)))));
+    q[4] = fm(qm, w[4], fm(ql, w[3], fm(hq, w[1], fm(qn, d, fm(H, s, ld(p, 4))))));
+  };
+  back(2, wl, L);
+  back(3, wh, Hs);
+  lf_flux<R>(L, Hs, nx, ny, nz, C, out);
 }
 
 // Flux through the same face with the linear upwind-biased 5th-order
@@ -402,13 +318,7 @@ __device__ __forceinline__ void face_flux_linear(const LD& ld, R nx, R ny, R nz,
     ql[n] = (R(2) * f0 - R(13) * f1 + R(47) * f2 + R(27) * f3 - R(3) * f4) * k60;
     qh[n] = (R(2) * f5 - R(13) * f4 + R(47) * f3 + R(27) * f2 - R(3) * f1) * k60;
   }
-  const R gam1 = C.gam1;
-  const R iL = rcp_(ql[0]), iH = rcp_(qh[0]);
-  const R Lu = ql[1] * iL, Lv = ql[2] * iL, Lw = ql[3] * iL;
-  const R Hu = qh[1] * iH, Hv = qh[2] * iH, Hw = qh[3] * iH;
-  const R Lp = gam1 * (ql[4] - R(0.5) * ql[0] * (Lu * Lu + Lv * Lv + Lw * Lw));
-  const R Hp = gam1 * (qh[4] - R(0.5) * qh[0] * (Hu * Hu + Hv * Hv + Hw * Hw));
-  lf_flux_prims<R>(ql[0], Lu, Lv, Lw, Lp, qh[0], Hu, Hv, Hw, Hp, nx, ny, nz, C, out);
+  lf_flux<R>(ql, qh, nx, ny, nz, C, out);
 }
 
 }  // namespace cbns
