@@ -163,6 +163,39 @@ int kchunk_default(int ntiles, int nint, int nsm) {
   return (nint + nchunk - 1) / nchunk;
 }
 
+// The chunk for a grid whose tiles at 8 planes a chunk or more make few waves of
+// CTAs: the least estimate of a launch's time in planes.  A chunk takes its
+// planes plus 0.7 for its start (the ring's first planes and the k-face below
+// it); while the CTAs fit the slots the launch is one chunk, beyond that the
+// work over the slots plus half a chunk of tail; CTAs alone on an SM run about
+// 1.5 times as fast as two.  Tiles cut by the grid's edge count by their
+// columns.  Measured us per step with this chunk against one of at least 8
+// planes: FP64 64x32x16 78 against 381 (8 CTAs marched the whole block while
+// 140 SMs idled), 97x61x45 245 against 272, 128x64x64 468 against 522; split
+// 64x32x16 69 against 258, 97x61x45 153 against 188; hybrid (3 per SM)
+// 64x32x16 146 against 277, 129x113x97 675 against 709.  Above about four
+// waves the chunks stay longer: at 193x161x129 4-plane chunks take 2770 us in
+// FP64 and 1618 split against 2682 and 1540 at 9.
+int kchunk_small(const Dims& d, int ntiles, int nsm, int per_sm) {
+  const int nint = d.KM - 2;
+  const double tiles = (d.IM - 2) * (d.JM - 2) / (double)(STAGE_TI * STAGE_TJ);
+  const double slots = (double)nsm * per_sm;
+  double best = 1e300;
+  int best_k = nint;
+  for (int kc = 1; kc <= nint; ++kc) {
+    const int nchunk = (nint + kc - 1) / kc;
+    const double items = (double)ntiles * nchunk, chunk = kc + 0.7;
+    const double cost = items <= nsm     ? chunk / 1.5
+                        : items <= slots ? chunk
+                                         : (std::max(1.0, tiles * nchunk / slots) + 0.5) * chunk;
+    if (cost < best - 1e-9) {
+      best = cost;
+      best_k = kc;
+    }
+  }
+  return best_k;
+}
+
 // Candidate chunkings for cbns_autotune at `per_sm` CTAs per SM (distinct values).
 std::vector<int> kchunk_candidates(const cbns_ctx* c, int per_sm) {
   const int ntiles = c->ntile_i * c->ntile_j, nint = c->d.KM - 2, slots = c->nsm * per_sm;
@@ -172,6 +205,7 @@ std::vector<int> kchunk_candidates(const cbns_ctx* c, int per_sm) {
   };
   for (double warm : {0.5, 2.0}) add(kchunk_by_waves(ntiles, nint, slots, warm));
   for (double waves : {4.0, 6.0, 9.0, 12.0}) add(kchunk_for_waves(ntiles, nint, slots, waves));
+  add(kchunk_small(c->d, ntiles, c->nsm, per_sm));
   return v;
 }
 
@@ -1127,21 +1161,14 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   // B200 for grids of a few million nodes: FP64 stages by TMA (about 10%
   // faster than the synchronous variant) and the split precision runs 2 CTAs
   // per SM, both with about 9 waves of CTAs; the hybrid runs 3 per SM (8%
-  // faster than 2) with chunks sized by the wave count and warm-up -- where
-  // that gives at least two full waves of CTAs; a smaller hybrid grid keeps 2
-  // per SM (its CTAs do not fill the GPU, and the 2-per-SM kernel holds more
-  // in registers)
+  // faster than 2) with chunks sized by the wave count and warm-up.  Where
+  // that makes fewer than four waves, the chunk of kchunk_small.
+  const bool hyb = p->precision == CBNS_PREC_HYBRID;
+  const int per_sm = hyb ? 3 : 2, slots = c->nsm * per_sm;
   c->stage_variant = p->precision == CBNS_PREC_SPLIT ? 0 : 1;
-  c->kchunk = kchunk_for_waves(ntiles, nint, c->nsm * 2, 9.0);
-  if (p->precision == CBNS_PREC_HYBRID) {
-    const int kc3 = kchunk_by_waves(ntiles, nint, c->nsm * 3, 0.5);
-    if ((long)ntiles * ((nint + kc3 - 1) / kc3) >= 2L * 3 * c->nsm) {
-      c->kchunk = kc3;
-    } else {
-      c->stage_variant = 0;
-      c->kchunk = kchunk_default(ntiles, nint, c->nsm);
-    }
-  }
+  c->kchunk = hyb ? kchunk_by_waves(ntiles, nint, slots, 0.5) : kchunk_for_waves(ntiles, nint, slots, 9.0);
+  if ((long)ntiles * ((nint + c->kchunk - 1) / c->kchunk) < 4L * slots)
+    c->kchunk = kchunk_small(d, ntiles, c->nsm, per_sm);
   stage_prepare();
   if (p->precision == CBNS_PREC_HYBRID) (void)weno_prepare();
   if (cudaStreamSynchronize(c->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess) {

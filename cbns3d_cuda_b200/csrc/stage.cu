@@ -55,7 +55,7 @@ namespace cbns {
 
 namespace {
 
-constexpr int TI = 16, TJ = 15, H = 3;
+constexpr int TI = STAGE_TI, TJ = STAGE_TJ, H = 3;
 constexpr int PW = TI + 2 * H;  // 22
 constexpr int PH = TJ + 2 * H;  // 21
 constexpr int NC = TI * TJ;     // 240 columns

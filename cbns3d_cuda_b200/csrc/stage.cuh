@@ -81,6 +81,7 @@ int weno_list_ctas(const Dims& d);
 cudaError_t launch_weno_list_batched(const ListArgs* args, const int* cta, int nblocks, int total, cudaStream_t s);
 // modes 1..3 only; hybrid: the StageArgs carry decision masks.
 cudaError_t launch_stage_batched(const BatchStage& b, int mode, bool visc, bool fp32, bool hybrid, cudaStream_t s);
+constexpr int STAGE_TI = 16, STAGE_TJ = 15;  // columns of a CTA's tile
 void stage_tiles(const Dims& d, int* ntile_i, int* ntile_j);
 
 }  // namespace cbns
