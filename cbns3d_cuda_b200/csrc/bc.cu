@@ -11,6 +11,8 @@
 //            copy of Q and primitives for every (i,j) (:417-492); (c) in
 //            inviscid runs, the spectral radius of every boundary node for the
 //            next time step (the boundary half of src/time_step_kernel.cu).
+// Without wake cut or wall (phase 2 has no work) one launch, bc_open, writes
+// what phases 1 and 3 write.
 // With CBNS_BC_FARFIELD (no counterpart in the reference) one kernel replaces
 // the three: boundary and ghost nodes keep their Q (a free-stream far field on
 // every face), only their primitives and spectral radii are formed; with
@@ -261,6 +263,107 @@ __global__ void bc_phase3(const BCArgs a) {
   if (!a.viscous && a.sigma) warp_sigma_max(a, sg, has);
 }
 
+// The reference's boundary conditions of a block without wake cut or wall
+// (i_begin = 1, i_end = 0) in one launch: the j = 0 and j = JM-1 rows then
+// hold their Q, so every value phases 1 and 3 write follows from interior
+// nodes and held rows alone -- a k-face node on an i face takes phase 1's
+// state, formed again from the interior node next to it -- and no thread reads
+// what another writes.  Threads, in order: the k faces (a side each, i
+// fastest), the j faces (spectral radii; viscous: primitives), the i faces
+// (four threads per (j, k) and side, one per written node: the three nodes
+// share a sector, which a thread per row wrote in 15 scattered stores).  Bound
+// by launch and load latency on small grids and by those scattered rows on
+// large ones.  Measured, the two launches -> this one: 64x32x16 9.6 -> 3.3 us,
+// 129x113x97 16.9 -> 8.2, 256x256x128 39 -> 30.
+__global__ void __launch_bounds__(128) bc_open(const BCArgs a) {
+  if (a.check_done && a.st->done) return;
+  const Dims& d = a.d;
+  const long VOL = d.VOL;
+  const long nK = (long)d.IM * d.JM, nJ = (long)d.IM * (d.KM - 2), nI = (long)(d.JM - 2) * (d.KM - 2);
+  long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const bool sigma = !a.viscous && a.sigma;
+  // Q and primitives an i-face node takes from the interior node at os (phase 1)
+  auto reset = [&](long os, double q[NEQ], PrimV& s) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) q[c] = a.q[c * VOL + os];
+    q[4] = a.p_inf / a.gam1 + 0.5 * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]) / q[0];
+    s.r = q[0];
+    s.u = q[1] / q[0];
+    s.v = q[2] / q[0];
+    s.w = q[3] / q[0];
+    s.p = a.gam1 * (q[4] - 0.5 * s.r * (s.u * s.u + s.v * s.v + s.w * s.w));
+  };
+  double sg = 0.0;
+  bool has = false;
+  if (e < 2 * nK) {
+    const int side = e >= nK;
+    const int r = (int)(side ? e - nK : e);
+    const int i = r % d.IM, j = r / d.IM;
+    const int src = side ? d.KM - 2 : 1, base = side ? d.KM - 1 : 0;
+    const long out = side ? d.PL : -d.PL;
+    double q[NEQ];
+    PrimV s;
+    if ((i == 0 || i == d.IM - 1) && j >= 1 && j <= d.JM - 2) {
+      reset(node_off(d, i == 0 ? 1 : d.IM - 2, j, src), q, s);
+    } else {
+      const long os = node_off(d, i, j, src);
+#pragma unroll
+      for (int c = 0; c < NEQ; ++c) q[c] = a.q[c * VOL + os];
+      s = prim_of(a.q, os, VOL, a.gam1);
+    }
+    const long o = node_off(d, i, j, base);
+#pragma unroll
+    for (int l = 0; l <= NG; ++l) {
+#pragma unroll
+      for (int c = 0; c < NEQ; ++c) a.q[c * VOL + o + l * out] = q[c];
+      if (a.viscous) put_prim(a, o + l * out, s);
+    }
+    if (sigma) {
+      sg = sigma_inv(a, o, s);
+      has = true;
+    }
+  } else if (e < 2 * (nK + nJ)) {
+    e -= 2 * nK;
+    const int side = e >= nJ;
+    const int r = (int)(side ? e - nJ : e);
+    const int i = r % d.IM, k = 1 + r / d.IM;
+    const long o = node_off(d, i, side ? d.JM - 1 : 0, k);
+    if (a.viscous) {
+      const PrimV s = prim_of(a.q, o, VOL, a.gam1);
+      put_prim(a, o, s);
+      if (side) {
+        put_prim(a, o + d.PX, s);
+      } else {
+        for (int l = 1; l <= NG; ++l) put_prim(a, o - l * d.PX, prim_of(a.q, o - l * d.PX, VOL, a.gam1));
+      }
+    } else if (sigma) {
+      sg = sigma_inv(a, o, prim_of(a.q, o, VOL, a.gam1));
+      has = true;
+    }
+  } else if (e < 2 * (nK + nJ) + 8 * nI) {
+    e -= 2 * (nK + nJ);
+    const int l = (int)(e & 3);
+    e >>= 2;
+    const int side = e >= nI;
+    const int r = (int)(side ? e - nI : e);
+    const int j = 1 + r % (d.JM - 2), k = 1 + r / (d.JM - 2);
+    double q[NEQ];
+    PrimV s;
+    reset(node_off(d, side ? d.IM - 2 : 1, j, k), q, s);
+    if (l <= NG) {
+      const long o = node_off(d, side ? d.IM - 1 + l : -l, j, k);
+#pragma unroll
+      for (int c = 0; c < NEQ; ++c) a.q[c * VOL + o] = q[c];
+      if (a.viscous) put_prim(a, o, s);
+      if (sigma && l == 0) {
+        sg = sigma_inv(a, o, s);
+        has = true;
+      }
+    }
+  }
+  if (sigma) warp_sigma_max(a, sg, has);
+}
+
 // Nodes of the ghosted box outside the interior (i, j, k in 1 .. N-2): the
 // six k planes of the outer slabs, then per interior k the six outer j rows,
 // then per interior (j, k) the six outer i nodes (x fastest where it can be).
@@ -491,15 +594,19 @@ cudaError_t launch_bc(const BCArgs& a, bool interior_prims, cudaStream_t s, int*
     if (launches) *launches += nl;
     return cudaGetLastError();
   }
-  bc_phase1<<<nblk(2L * (d.JM - 2) * (d.KM - 2), B), B, 0, s>>>(a);
-  ++nl;
   // phase 2 has work only if some i takes the wake or the wall branch
   const bool wake_any = (a.i_begin - 1u) > 0u;  // i = 0 satisfies i_begin-1 > i
   const bool wall_any = a.i_end > 0u;
-  if (wake_any || wall_any) {
-    bc_phase2<<<nblk((long)d.IM * (d.KM - 2), B), B, 0, s>>>(a);
+  if (!wake_any && !wall_any) {
+    const long n = 2L * d.IM * d.JM + 2L * d.IM * (d.KM - 2) + 8L * (d.JM - 2) * (d.KM - 2);
+    bc_open<<<nblk(n, B), B, 0, s>>>(a);
     ++nl;
+    if (launches) *launches += nl;
+    return cudaGetLastError();
   }
+  bc_phase1<<<nblk(2L * (d.JM - 2) * (d.KM - 2), B), B, 0, s>>>(a);
+  bc_phase2<<<nblk((long)d.IM * (d.KM - 2), B), B, 0, s>>>(a);
+  nl += 2;
   bc_phase3<<<nblk(n3, B), B, 0, s>>>(a);
   ++nl;
   if (launches) *launches += nl;
