@@ -46,6 +46,7 @@ struct cbns_ctx {
   Dims d;
   cudaStream_t own = nullptr, stream = nullptr;
   double* qb[3] = {nullptr, nullptr, nullptr};
+  float* q32[3] = {nullptr, nullptr, nullptr};  // FP32-flux precisions: the buffers' FP32 copies
   int lq = 0, lp = 1, ls = 2;  // physical index of logical Q, Q_p, spare
   Fields f;
   double* staging = nullptr;
@@ -67,7 +68,8 @@ struct cbns_ctx {
   int ntile_i = 1, ntile_j = 1, kchunk = 1;
   int stage_variant = 0;  // compiled variant of the stage kernel (set in cbns_create, cbns_autotune)
   int nsm = 148;          // SMs of the device
-  StageMaps tm[3];        // FP32 precisions: TMA maps of the stage kernel, per state buffer
+  StageMaps tm[3];        // TMA maps of the stage kernel, per state buffer as the stage input
+  CUtensorMap tm_rk[3];   // per state buffer, its box as an RK operand
   // hybrid flux: the learned sensor's parameters and per-face decisions
   float* sensor_params = nullptr;  // device, CBNS_SENSOR_NPARAM floats
   unsigned char* mask = nullptr;   // device, one byte per face: the decisions the fluxes use
@@ -247,6 +249,13 @@ void fill_met(const cbns_ctx* c, const double* out[10]) {
   for (int m = 0; m < 10; ++m) out[m] = c->f.met[m];
 }
 
+// The FP32 copy of a state buffer (null: a precision without, or another array).
+float* copy32(const cbns_ctx* c, const double* q) {
+  for (int b = 0; b < 3; ++b)
+    if (q == c->qb[b]) return c->q32[b];
+  return nullptr;
+}
+
 BCArgs bc_args(cbns_ctx* c, double* q, bool check_done, bool sigma) {
   BCArgs a;
   a.d = c->d;
@@ -258,6 +267,7 @@ BCArgs bc_args(cbns_ctx* c, double* q, bool check_done, bool sigma) {
   a.i_end = c->ph.i_end;
   a.viscous = c->ph.viscous;
   a.q = q;
+  a.q32 = copy32(c, q);
   fill_met(c, a.met);
   for (int m = 0; m < 6; ++m) a.prim[m] = c->f.prim[m];
   a.st = c->st;
@@ -320,10 +330,16 @@ StageArgs stage_args(cbns_ctx* c, const double* src, const double* q0, const dou
   a.sigma = sigma;
   a.mask = c->ph.precision == CBNS_PREC_HYBRID ? c->mask : nullptr;
   a.wflux = c->wflux;
-  a.tm = c->tm[0];  // src is always one of the three state buffers
+  a.tm = c->tm[0];  // src, q0 and qp are state buffers (or q0, qp null: RHS only)
   for (int b = 0; b < 3; ++b)
     if (src == c->qb[b]) a.tm = c->tm[b];
-  for (int m = 0; m < 6; ++m) a.area32[m] = c->f.area32[m];
+  for (int b = 0; b < 3; ++b) {
+    if (q0 == c->qb[b]) a.tm.q0 = c->tm_rk[b];
+    if (qp == c->qb[b]) a.tm.qp = c->tm_rk[b];
+  }
+  a.src32 = copy32(c, src);
+  a.out32 = copy32(c, out);
+  for (int m = 0; m < 9; ++m) a.area32[m] = c->f.area32[m];
   return a;
 }
 
@@ -390,6 +406,10 @@ int replicate_q(cbns_ctx* c) {
   const size_t bytes = (size_t)NEQ * c->d.VOL * sizeof(double);
   for (int b = 0; b < 3; ++b)
     if (b != c->lq) CK(cudaMemcpyAsync(c->qb[b], c->qb[c->lq], bytes, cudaMemcpyDeviceToDevice, c->stream));
+  if (c->q32[0]) {
+    CK(launch_narrow_state(c->d, c->qb[c->lq], c->q32, c->stream));
+    c->launches += 1;
+  }
   return CBNS_OK;
 }
 
@@ -418,8 +438,8 @@ SensorSet sensor_set(cbns_ctx* c, const double* q, bool check_done, bool every_s
   m.d = c->d;
   m.gamma = (float)c->ph.gamma;
   m.gam1 = (float)c->ph.gam1;
-  m.q = q;
-  for (int k = 0; k < 10; ++k) m.area[k] = c->f.area[k];
+  m.q = copy32(c, q);
+  for (int k = 0; k < 9; ++k) m.area[k] = c->f.area32[k];
   m.params = c->sensor_params;
   m.tau = c->sensor_tau;
   m.every = every;
@@ -1050,20 +1070,29 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
     if (rc == CBNS_OK)
       for (int m = 0; m < 10; ++m) c->f.area[m] = tmp + (size_t)m * d.VOL;
   }
-  for (int m = 0; m < 6; ++m) c->f.area32[m] = nullptr;
-  if (p->precision != CBNS_PREC_FP64) {
-    // one allocation, components VOL floats apart (one 4-D tensor map covers them)
+  for (int m = 0; m < 9; ++m) c->f.area32[m] = nullptr;
+  const bool fp32 = p->precision != CBNS_PREC_FP64;
+  if (fp32) {
+    // one allocation, components VOL floats apart (one 4-D tensor map covers
+    // them); the same for each state buffer's FP32 copy
     double* tmp = nullptr;
-    rc = rc == CBNS_OK ? dalloc(c, &tmp, (size_t)3 * d.VOL) : rc;
+    rc = rc == CBNS_OK ? dalloc(c, &tmp, (size_t)9 * d.VOL / 2) : rc;
     if (rc == CBNS_OK)
-      for (int m = 0; m < 6; ++m) c->f.area32[m] = reinterpret_cast<float*>(tmp) + (size_t)m * d.VOL;
+      for (int m = 0; m < 9; ++m) c->f.area32[m] = reinterpret_cast<float*>(tmp) + (size_t)m * d.VOL;
+    for (int b = 0; b < 3 && rc == CBNS_OK; ++b) {
+      rc = dalloc(c, &tmp, (size_t)NEQ * d.VOL / 2);
+      c->q32[b] = reinterpret_cast<float*>(tmp);
+    }
   }
   for (int m = 0; m < 7 && rc == CBNS_OK; ++m) rc = dalloc(c, &c->f.prim[m], d.VOL);
   for (int m = 0; m < 12; ++m) c->f.vflux[m] = nullptr;
   for (int m = 0; m < 4; ++m) c->f.dfv[m] = nullptr;
   if (p->viscous) {
     for (int m = 0; m < 12 && rc == CBNS_OK; ++m) rc = dalloc(c, &c->f.vflux[m], d.VOL);
-    for (int m = 0; m < 4 && rc == CBNS_OK; ++m) rc = dalloc(c, &c->f.dfv[m], d.VOL);
+    // one allocation (one 4-D tensor map covers its FP32 elements)
+    double* tmp = nullptr;
+    rc = rc == CBNS_OK ? dalloc(c, &tmp, (size_t)4 * d.VOL) : rc;
+    for (int m = 0; m < 4 && rc == CBNS_OK; ++m) c->f.dfv[m] = tmp + (size_t)m * d.VOL;
   }
   const long NGt = (long)d.IG * d.JG * d.KG;
   c->staging_elems = (size_t)std::max(5 * NGt, 10L * d.IM * d.JM * d.KM);
@@ -1113,22 +1142,23 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   }
   c->stream = c->own;
   {
-    // the stage kernels' TMA boxes (stage.cu), per state buffer
+    // the stage kernels' TMA boxes (stage.cuh), per state buffer
     bool ok = true;
-    const bool fp32 = p->precision != CBNS_PREC_FP64;
     for (int b = 0; b < 3; ++b) {
       StageMaps& m = c->tm[b];
-      if (fp32) {  // halo boxes of the state, FP32 area vectors
-        ok = ok && encode_node_map(&m.q_a, c->qb[b], 8, d.PX, d.JG, d.KG, d.VOL, NEQ, 4, 15, NEQ);
-        ok = ok && encode_node_map(&m.q_b, c->qb[b], 8, d.PX, d.JG, d.KG, d.VOL, NEQ, 16, 3, NEQ);
-        ok = ok && encode_node_map(&m.xi, c->f.area32[0], 4, d.PX, d.JG, d.KG, d.VOL, 6, 24, 15, 3);
-        ok = ok && encode_node_map(&m.eta, c->f.area32[0], 4, d.PX, d.JG, d.KG, d.VOL, 6, 16, 17, 3);
-      } else {  // ring column and plane boxes of the state, FP64 area vectors
-        ok = ok && encode_node_map(&m.q_a, c->qb[b], 8, d.PX, d.JG, d.KG, d.VOL, NEQ, 16, 15, NEQ);
-        ok = ok && encode_node_map(&m.q_b, c->qb[b], 8, d.PX, d.JG, d.KG, d.VOL, NEQ, 24, 21, NEQ);
-        ok = ok && encode_node_map(&m.xi, c->f.area[0], 8, d.PX, d.JG, d.KG, d.VOL, 10, 24, 15, 3);
-        ok = ok && encode_node_map(&m.eta, c->f.area[0], 8, d.PX, d.JG, d.KG, d.VOL, 10, 16, 17, 3);
-      }
+      const void *q = fp32 ? (const void*)c->q32[b] : c->qb[b], *ar = fp32 ? (const void*)c->f.area32[0] : c->f.area[0];
+      const int es = fp32 ? 4 : 8, na = fp32 ? 9 : 10;
+      ok = ok && encode_node_map(&m.q_a, q, es, d.PX, d.JG, d.KG, d.VOL, NEQ, 16, 15, NEQ);
+      ok = ok && encode_node_map(&m.q_b, q, es, d.PX, d.JG, d.KG, d.VOL, NEQ, 24, 21, NEQ);
+      ok = ok && encode_node_map(&m.xi, ar, es, d.PX, d.JG, d.KG, d.VOL, na, 24, 15, 3);
+      ok = ok && encode_node_map(&m.eta, ar, es, d.PX, d.JG, d.KG, d.VOL, na, 16, 17, 3);
+      ok = ok && encode_node_map(&m.zeta, ar, es, d.PX, d.JG, d.KG, d.VOL, na, 16, 15, 3);
+      ok = ok && encode_node_map(&c->tm_rk[b], c->qb[b], 8, d.PX, d.JG, d.KG, d.VOL, NEQ, 16, 15, NEQ);
+      ok = ok && encode_node_map(&m.iJ, c->f.area[0], 8, d.PX, d.JG, d.KG, d.VOL, 10, 16, 15, 1);
+      m.q0 = m.qp = c->tm_rk[b];
+      m.dfv = m.iJ;  // FP32 kernels of viscous runs only
+      if (p->viscous && fp32)  // FP32 elements in arrays VOL doubles apart
+        ok = ok && encode_node_map(&m.dfv, c->f.dfv[0], 4, d.PX, d.JG, d.KG, 2 * d.VOL, 4, 16, 15, 4);
     }
     if (!ok) {
       g_last = "cuTensorMapEncodeTiled refused the stage kernel's tensor maps";
@@ -1141,8 +1171,10 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   for (int b = 0; b < 3; ++b) cudaMemsetAsync(c->qb[b], 0, (size_t)NEQ * d.VOL * sizeof(double), c->stream);
   for (int m = 0; m < 10; ++m) cudaMemsetAsync(c->f.met[m], 0, d.VOL * sizeof(double), c->stream);
   for (int m = 0; m < 10; ++m) cudaMemsetAsync(c->f.area[m], 0, d.VOL * sizeof(double), c->stream);
-  for (int m = 0; m < 6; ++m)
+  for (int m = 0; m < 9; ++m)
     if (c->f.area32[m]) cudaMemsetAsync(c->f.area32[m], 0, d.VOL * sizeof(float), c->stream);
+  for (int b = 0; b < 3; ++b)
+    if (c->q32[b]) cudaMemsetAsync(c->q32[b], 0, (size_t)NEQ * d.VOL * sizeof(float), c->stream);
   for (int m = 0; m < 7; ++m) cudaMemsetAsync(c->f.prim[m], 0, d.VOL * sizeof(double), c->stream);
   if (p->viscous) {
     for (int m = 0; m < 12; ++m) cudaMemsetAsync(c->f.vflux[m], 0, d.VOL * sizeof(double), c->stream);
@@ -1163,13 +1195,13 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   // per SM, both with about 9 waves of CTAs; the hybrid runs 3 per SM (8%
   // faster than 2) with chunks sized by the wave count and warm-up.  Where
   // that makes fewer than four waves, the chunk of kchunk_small.
-  const bool hyb = p->precision == CBNS_PREC_HYBRID;
-  const int per_sm = hyb ? 3 : 2, slots = c->nsm * per_sm;
-  c->stage_variant = p->precision == CBNS_PREC_SPLIT ? 0 : 1;
-  c->kchunk = hyb ? kchunk_by_waves(ntiles, nint, slots, 0.5) : kchunk_for_waves(ntiles, nint, slots, 9.0);
+  const int per_sm = fp32 ? 3 : 2, slots = c->nsm * per_sm;
+  c->stage_variant = 1;
+  c->kchunk = fp32 ? kchunk_by_waves(ntiles, nint, slots, 0.5) : kchunk_for_waves(ntiles, nint, slots, 9.0);
   if ((long)ntiles * ((nint + c->kchunk - 1) / c->kchunk) < 4L * slots)
     c->kchunk = kchunk_small(d, ntiles, c->nsm, per_sm);
-  stage_prepare();
+  if (fp32) stage32_prepare();
+  else stage_prepare();
   if (p->precision == CBNS_PREC_HYBRID) (void)weno_prepare();
   if (cudaStreamSynchronize(c->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     g_last = "context initialisation failed";
@@ -1697,6 +1729,7 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
   float best_ms = 0.f;
   rc = time_it(v0, kc0, &best_ms);
   for (int v = 0; v < nv && rc == CBNS_OK; ++v) {
+    if (fp32 && v == 2) continue;  // variant 1's kernel again
     // FP32 variant v runs 2 + v CTAs per SM, the FP64 ones 2; each with its candidate k chunks
     for (int kc : kchunk_candidates(c, fp32 ? 2 + v : 2)) {
       if (v == v0 && kc == kc0) continue;

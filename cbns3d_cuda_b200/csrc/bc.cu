@@ -31,6 +31,12 @@ namespace cbns {
 
 namespace {
 
+// variable c of node offset o: Q and, where there is one, its FP32 copy
+__device__ __forceinline__ void put_q(const BCArgs& a, int c, long o, double v) {
+  a.q[c * a.d.VOL + o] = v;
+  if (a.q32) a.q32[c * a.d.VOL + o] = (float)v;
+}
+
 struct PrimV {
   double r, u, v, w, p;
 };
@@ -108,11 +114,11 @@ __global__ void bc_phase1(const BCArgs a) {
   s.p = a.gam1 * (E - 0.5 * s.r * (s.u * s.u + s.v * s.v + s.w * s.w));
   for (int l = 0; l <= NG; ++l) {
     const long o = node_off(d, base + dir * l, j, k);
-    a.q[o] = rr;
-    a.q[VOL + o] = ru;
-    a.q[2 * VOL + o] = rv;
-    a.q[3 * VOL + o] = rw;
-    a.q[4 * VOL + o] = E;
+    put_q(a, 0, o, rr);
+    put_q(a, 1, o, ru);
+    put_q(a, 2, o, rv);
+    put_q(a, 3, o, rw);
+    put_q(a, 4, o, E);
     if (a.viscous) put_prim(a, o, s);
   }
 }
@@ -139,16 +145,16 @@ __global__ void bc_phase2(const BCArgs a) {
     const long o0 = node_off(d, i, 0, k), m0 = node_off(d, m, 0, k);
 #pragma unroll
     for (int c = 0; c < NEQ; ++c) {
-      q[c * VOL + o0] = v5[c];
-      q[c * VOL + m0] = v5[c];
+      put_q(a, c, o0, v5[c]);
+      put_q(a, c, m0, v5[c]);
     }
     for (int l = 1; l <= NG; ++l) {
       const long a1 = node_off(d, m, l, k), b1 = node_off(d, i, -l, k);
       const long a2 = node_off(d, i, l, k), b2 = node_off(d, m, -l, k);
 #pragma unroll
       for (int c = 0; c < NEQ; ++c) {
-        q[c * VOL + b1] = q[c * VOL + a1];
-        q[c * VOL + b2] = q[c * VOL + a2];
+        put_q(a, c, b1, q[c * VOL + a1]);
+        put_q(a, c, b2, q[c * VOL + a2]);
       }
     }
   } else if (a.i_end > ui) {
@@ -157,18 +163,18 @@ __global__ void bc_phase2(const BCArgs a) {
       // adiabatic no-slip wall
       const double rr = q[o1], ru = q[VOL + o1], rv = q[2 * VOL + o1], rw = q[3 * VOL + o1], rE = q[4 * VOL + o1];
       const double pp = gam1 * (rE - 0.5 * (ru * ru + rv * rv + rw * rw) / rr);
-      q[o0] = rr;
-      q[VOL + o0] = 0.0;
-      q[2 * VOL + o0] = 0.0;
-      q[3 * VOL + o0] = 0.0;
-      q[4 * VOL + o0] = pp / gam1;
+      put_q(a, 0, o0, rr);
+      put_q(a, 1, o0, 0.0);
+      put_q(a, 2, o0, 0.0);
+      put_q(a, 3, o0, 0.0);
+      put_q(a, 4, o0, pp / gam1);
       for (int l = 1; l <= NG; ++l) {
         const long s1 = node_off(d, i, l, k), g1 = node_off(d, i, -l, k);
-        q[g1] = q[s1];
-        q[VOL + g1] = -q[VOL + s1];
-        q[2 * VOL + g1] = -q[2 * VOL + s1];
-        q[3 * VOL + g1] = -q[3 * VOL + s1];
-        q[4 * VOL + g1] = q[4 * VOL + s1];
+        put_q(a, 0, g1, q[s1]);
+        put_q(a, 1, g1, -q[VOL + s1]);
+        put_q(a, 2, g1, -q[2 * VOL + s1]);
+        put_q(a, 3, g1, -q[3 * VOL + s1]);
+        put_q(a, 4, g1, q[4 * VOL + s1]);
       }
     } else {
       // slip wall, tangent in the x-y plane
@@ -185,20 +191,20 @@ __global__ void bc_phase2(const BCArgs a) {
         const double a0 = q[s1], a1 = q[VOL + s1], a2 = q[2 * VOL + s1], a3 = q[3 * VOL + s1], a4 = q[4 * VOL + s1];
         const double vt = a1 * tx + a2 * ty;
         const double b1 = 2 * vt * tx - a1, b2 = 2 * vt * ty - a2;
-        q[g1] = a0;
-        q[VOL + g1] = b1;
-        q[2 * VOL + g1] = b2;
-        q[3 * VOL + g1] = a3;
+        put_q(a, 0, g1, a0);
+        put_q(a, 1, g1, b1);
+        put_q(a, 2, g1, b2);
+        put_q(a, 3, g1, a3);
         // the reference's energy expression, sign of the last term included
-        q[4 * VOL + g1] = a4 - 0.5 * (a1 * a1 + a2 * a2 - b1 * b1 + b2 * b2) / a0;
+        put_q(a, 4, g1, a4 - 0.5 * (a1 * a1 + a2 * a2 - b1 * b1 + b2 * b2) / a0);
       }
       const double vt = s.u * tx + s.v * ty;
       const double uu = vt * tx, vv = vt * ty;
-      q[o0] = s.r;
-      q[VOL + o0] = s.r * uu;
-      q[2 * VOL + o0] = s.r * vv;
-      q[3 * VOL + o0] = s.r * s.w;
-      q[4 * VOL + o0] = s.p / gam1 + 0.5 * s.r * (uu * uu + vv * vv + s.w * s.w);
+      put_q(a, 0, o0, s.r);
+      put_q(a, 1, o0, s.r * uu);
+      put_q(a, 2, o0, s.r * vv);
+      put_q(a, 3, o0, s.r * s.w);
+      put_q(a, 4, o0, s.p / gam1 + 0.5 * s.r * (uu * uu + vv * vv + s.w * s.w));
     }
   }
 }
@@ -248,7 +254,7 @@ __global__ void bc_phase3(const BCArgs a) {
       for (int l = 0; l <= NG; ++l) {
         const long o = node_off(d, i, j, base + dir * l);
 #pragma unroll
-        for (int c = 0; c < NEQ; ++c) a.q[c * VOL + o] = v5[c];
+        for (int c = 0; c < NEQ; ++c) put_q(a, c, o, v5[c]);
       }
       const PrimV s = prim_of(a.q, os, VOL, gam1);
       if (a.viscous) {
@@ -273,20 +279,23 @@ __global__ void bc_phase3(const BCArgs a) {
 // (four threads per (j, k) and side, one per written node: the three nodes
 // share a sector, which a thread per row wrote in 15 scattered stores).  Bound
 // by launch and load latency on small grids and by those scattered rows on
-// large ones.  Measured, the two launches -> this one: 64x32x16 9.6 -> 3.3 us,
-// 129x113x97 16.9 -> 8.2, 256x256x128 39 -> 30.
+// large ones.  Measured, the two launches -> this one: 64x32x16 9.6 -> 2.4 us
+// (4.1 with the spectral radii), 97x61x45 11.8 -> 2.8 (7.8), 256x256x128 39 ->
+// 22 (46).  With an FP32 copy to write the scattered rows cost as much again
+// (43 and 68 us).
+template <bool VISC, bool SIGMA>
 __global__ void __launch_bounds__(128) bc_open(const BCArgs a) {
   if (a.check_done && a.st->done) return;
   const Dims& d = a.d;
   const long VOL = d.VOL;
   const long nK = (long)d.IM * d.JM, nJ = (long)d.IM * (d.KM - 2), nI = (long)(d.JM - 2) * (d.KM - 2);
   long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const bool sigma = !a.viscous && a.sigma;
-  // Q and primitives an i-face node takes from the interior node at os (phase 1)
+  // Q and (where wanted) primitives an i-face node takes from the interior node at os (phase 1)
   auto reset = [&](long os, double q[NEQ], PrimV& s) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) q[c] = a.q[c * VOL + os];
     q[4] = a.p_inf / a.gam1 + 0.5 * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]) / q[0];
+    if (!VISC && !SIGMA) return;
     s.r = q[0];
     s.u = q[1] / q[0];
     s.v = q[2] / q[0];
@@ -309,16 +318,16 @@ __global__ void __launch_bounds__(128) bc_open(const BCArgs a) {
       const long os = node_off(d, i, j, src);
 #pragma unroll
       for (int c = 0; c < NEQ; ++c) q[c] = a.q[c * VOL + os];
-      s = prim_of(a.q, os, VOL, a.gam1);
+      if (VISC || SIGMA) s = prim_of(a.q, os, VOL, a.gam1);
     }
     const long o = node_off(d, i, j, base);
 #pragma unroll
     for (int l = 0; l <= NG; ++l) {
 #pragma unroll
-      for (int c = 0; c < NEQ; ++c) a.q[c * VOL + o + l * out] = q[c];
-      if (a.viscous) put_prim(a, o + l * out, s);
+      for (int c = 0; c < NEQ; ++c) put_q(a, c, o + l * out, q[c]);
+      if (VISC) put_prim(a, o + l * out, s);
     }
-    if (sigma) {
+    if (SIGMA) {
       sg = sigma_inv(a, o, s);
       has = true;
     }
@@ -328,7 +337,7 @@ __global__ void __launch_bounds__(128) bc_open(const BCArgs a) {
     const int r = (int)(side ? e - nJ : e);
     const int i = r % d.IM, k = 1 + r / d.IM;
     const long o = node_off(d, i, side ? d.JM - 1 : 0, k);
-    if (a.viscous) {
+    if (VISC) {
       const PrimV s = prim_of(a.q, o, VOL, a.gam1);
       put_prim(a, o, s);
       if (side) {
@@ -336,7 +345,7 @@ __global__ void __launch_bounds__(128) bc_open(const BCArgs a) {
       } else {
         for (int l = 1; l <= NG; ++l) put_prim(a, o - l * d.PX, prim_of(a.q, o - l * d.PX, VOL, a.gam1));
       }
-    } else if (sigma) {
+    } else if (SIGMA) {
       sg = sigma_inv(a, o, prim_of(a.q, o, VOL, a.gam1));
       has = true;
     }
@@ -353,15 +362,15 @@ __global__ void __launch_bounds__(128) bc_open(const BCArgs a) {
     if (l <= NG) {
       const long o = node_off(d, side ? d.IM - 1 + l : -l, j, k);
 #pragma unroll
-      for (int c = 0; c < NEQ; ++c) a.q[c * VOL + o] = q[c];
-      if (a.viscous) put_prim(a, o, s);
-      if (sigma && l == 0) {
+      for (int c = 0; c < NEQ; ++c) put_q(a, c, o, q[c]);
+      if (VISC) put_prim(a, o, s);
+      if (SIGMA && l == 0) {
         sg = sigma_inv(a, o, s);
         has = true;
       }
     }
   }
-  if (sigma) warp_sigma_max(a, sg, has);
+  if (SIGMA) warp_sigma_max(a, sg, has);
 }
 
 // Nodes of the ghosted box outside the interior (i, j, k in 1 .. N-2): the
@@ -508,7 +517,7 @@ __global__ void bc_characteristic(const BCArgs a, int dir, int side0, int nsides
 #pragma unroll
   for (int l = 0; l <= NG; ++l)
 #pragma unroll
-    for (int m = 0; m < 5; ++m) q[m * VOL + ob + l * out] = qb[m];
+    for (int m = 0; m < 5; ++m) put_q(a, m, ob + l * out, qb[m]);
 }
 
 // CBNS_BC_OGRID, last pass: every node with i < wrap or i >= IM - wrap, the
@@ -530,7 +539,7 @@ __global__ void bc_wrap(const BCArgs a) {
   const long o = node_off(d, i, j, k), os = node_off(d, src, j, k);
   const long VOL = d.VOL;
 #pragma unroll
-  for (int c = 0; c < NEQ; ++c) a.q[c * VOL + o] = a.q[c * VOL + os];
+  for (int c = 0; c < NEQ; ++c) put_q(a, c, o, a.q[c * VOL + os]);
   if (a.viscous) {
 #pragma unroll
     for (int m = 0; m < 6; ++m) a.prim[m][o] = a.prim[m][os];
@@ -599,7 +608,9 @@ cudaError_t launch_bc(const BCArgs& a, bool interior_prims, cudaStream_t s, int*
   const bool wall_any = a.i_end > 0u;
   if (!wake_any && !wall_any) {
     const long n = 2L * d.IM * d.JM + 2L * d.IM * (d.KM - 2) + 8L * (d.JM - 2) * (d.KM - 2);
-    bc_open<<<nblk(n, B), B, 0, s>>>(a);
+    if (a.viscous) bc_open<true, false><<<nblk(n, B), B, 0, s>>>(a);
+    else if (a.sigma) bc_open<false, true><<<nblk(n, B), B, 0, s>>>(a);
+    else bc_open<false, false><<<nblk(n, B), B, 0, s>>>(a);
     ++nl;
     if (launches) *launches += nl;
     return cudaGetLastError();

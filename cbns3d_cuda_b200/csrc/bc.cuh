@@ -11,6 +11,7 @@ struct BCArgs {
   unsigned i_begin, i_end;
   int viscous;
   double* q;             // the buffer the boundary conditions act on (5 fields)
+  float* q32;            // its FP32 copy (FP32-flux precisions, else null)
   const double* met[10];
   double* prim[6];       // rho,u,v,w,p,T (viscous runs)
   StepState* st;

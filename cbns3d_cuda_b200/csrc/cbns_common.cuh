@@ -46,7 +46,7 @@ struct Phys {
 struct Fields {
   double* met[10];   // xi_x, xi_y, xi_z, eta_x, eta_y, eta_z, zeta_x, zeta_y, zeta_z, Jac
   double* area[10];  // J*grad(xi) (3), J*grad(eta) (3), J*grad(zeta) (3), 1/J
-  float* area32[6];  // FP32 and hybrid contexts: J*grad(xi), J*grad(eta) rounded to FP32
+  float* area32[9];  // FP32-flux contexts: J*grad(xi), J*grad(eta), J*grad(zeta) rounded to FP32
   double* prim[7];   // rho, u, v, w, p, T, mu (viscous upkeep; on-demand otherwise)
   double* vflux[12]; // E0..E3, F0..F3, G0..G3 (viscous node fluxes, times J-scaled normals)
   double* dfv[4];    // divergence of the viscous node fluxes at the interior nodes (momentum 3, energy)

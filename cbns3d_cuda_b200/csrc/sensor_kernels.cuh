@@ -25,8 +25,8 @@ struct SampleArgs {
 struct MaskArgs {
   Dims d;
   float gamma, gam1;
-  const double* q;
-  const double* area[10];
+  const float* q;           // the state's FP32 copy (5 fields)
+  const float* area[9];     // node area vectors in FP32
   const float* params;      // CBNS_SENSOR_NPARAM floats (device)
   float tau;
   unsigned every;           // evaluate on steps with steps % every == 1 % every (1: always)

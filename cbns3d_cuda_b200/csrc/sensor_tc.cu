@@ -71,11 +71,11 @@ struct RowSmem {
 // KB of ring; four slots and 4 CTAs per SM measured 2% slower).
 constexpr int SW_D = 2;
 struct WinSmem {
-  double v[SW_D][8][SW_T];
+  float v[SW_D][8][SW_T];
 };
 
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tc::smem_u32(smem)), "l"(gmem) : "memory");
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(tc::smem_u32(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_ring() {
@@ -124,13 +124,11 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
   const float gamma = a.gamma, gam1 = a.gam1;
   bool ok = true;
 
-  auto load_q = [&](const double* p, double q[5]) {
+  auto load_q = [&](const float* p, float q[5]) {
 #pragma unroll
     for (int n = 0; n < 5; ++n) q[n] = __ldg(p + n * VOL);
   };
-  auto prim_of = [&](const double q[5]) {
-    return node_prim((float)q[0], (float)q[1], (float)q[2], (float)q[3], (float)q[4], gam1);
-  };
+  auto prim_of = [&](const float q[5]) { return node_prim(q[0], q[1], q[2], q[3], q[4], gam1); };
 
   float f[SN_IN];
   if (KIND == 0) {  // i-faces, row by row
@@ -140,7 +138,7 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
     // this thread's share of a row: node x = t (and x = SW_T + t for t < 5)
     // and the area vector of node x = t (and x = SW_T for t = 0); the next
     // row's share is loaded while the current row goes through the network
-    double q0[5], q1[5], a0[3], a1[3];
+    float q0[5], q1[5], a0[3], a1[3];
     auto fetch = [&](int r) {
       const int j = 1 + r % (JM - 2), k = 1 + r / (JM - 2);
       const int ia = i0 - 2 + t, ib = i0 - 2 + SW_T + t;
@@ -157,7 +155,7 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
         for (int m = 0; m < 3; ++m) a1[m] = __ldg(a.area[m] + o);
       }
     };
-    auto put = [&](int x, const double q[5]) {
+    auto put = [&](int x, const float q[5]) {
       const NodePrim p = prim_of(q);
       rs.pr[0][x] = p.r;
       rs.pr[1][x] = p.p;
@@ -173,11 +171,11 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
       if (t < 5 && i0 - 2 + SW_T + t <= IM + 1) put(SW_T + t, q1);
       if (i0 + t <= IM + 1) {
 #pragma unroll
-        for (int m = 0; m < 3; ++m) rs.ax[m][t] = (float)a0[m];
+        for (int m = 0; m < 3; ++m) rs.ax[m][t] = a0[m];
       }
       if (t == 0 && i0 + SW_T <= IM + 1) {
 #pragma unroll
-        for (int m = 0; m < 3; ++m) rs.ax[m][SW_T] = (float)a1[m];
+        for (int m = 0; m < 3; ++m) rs.ax[m][SW_T] = a1[m];
       }
       if (r + 1 < r1) fetch(r + 1);
       __syncthreads();
@@ -231,16 +229,16 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
         const int slot = u % SW_D;
         const long on = obase + (long)(f0 + 3 + u) * sd, oa = obase + (long)(f0 + 1 + u) * sd;
 #pragma unroll
-        for (int n = 0; n < 5; ++n) cp_async8(&ws.v[slot][n][t], a.q + n * VOL + on);
+        for (int n = 0; n < 5; ++n) cp_async4(&ws.v[slot][n][t], a.q + n * VOL + on);
 #pragma unroll
-        for (int m = 0; m < 3; ++m) cp_async8(&ws.v[slot][5 + m][t], a.area[am + m] + oa);
+        for (int m = 0; m < 3; ++m) cp_async4(&ws.v[slot][5 + m][t], a.area[am + m] + oa);
       }
       cp_async_commit();  // one group per step, empty or not
     };
 #pragma unroll
     for (int u = 0; u < SW_D; ++u) issue(u);
     if (valid) {
-      double qq[5];
+      float qq[5];
       load_q(a.q + obase + (long)(f0 - 2) * sd, qq);
       W0 = prim_of(qq);
       load_q(a.q + obase + (long)(f0 - 1) * sd, qq);
@@ -252,7 +250,7 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
       load_q(a.q + obase + (long)(f0 + 2) * sd, qq);
       W4 = prim_of(qq);
 #pragma unroll
-      for (int m = 0; m < 3; ++m) Aa[m] = (float)__ldg(a.area[am + m] + obase + (long)f0 * sd);
+      for (int m = 0; m < 3; ++m) Aa[m] = __ldg(a.area[am + m] + obase + (long)f0 * sd);
     }
     // One face: the window (w0..w4 hold positions fc-2..fc+2, wn receives
     // fc+3), the area vectors of positions fc (A0) and fc+1 (A1 receives).
@@ -263,12 +261,12 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
       cp_async_wait_ring();  // the copies of step u have landed
       if (valid) {
         const int slot = u % SW_D;
-        double nq[5];
+        float nq[5];
 #pragma unroll
         for (int n = 0; n < 5; ++n) nq[n] = ws.v[slot][n][t];
         wn = prim_of(nq);
 #pragma unroll
-        for (int m = 0; m < 3; ++m) A1[m] = (float)ws.v[slot][5 + m][t];
+        for (int m = 0; m < 3; ++m) A1[m] = ws.v[slot][5 + m][t];
       }
       issue(u + SW_D);  // refill the slot just read
       if (valid) {

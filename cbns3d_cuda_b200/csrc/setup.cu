@@ -96,10 +96,10 @@ __global__ void metrics_ghosts(Dims d, Met M) {
 // Node area vectors J*grad(xi), J*grad(eta), J*grad(zeta) and 1/J over the
 // ghosted box: the face normal of the reference is the mean of the two nodes'
 // J*grad(xi) (src/rec_riemann_kernel.cu:44-49), so it is formed once here.
-// The FP32 kernels stage FP32 copies of J*grad(xi) and J*grad(eta) (A32, may
-// be absent).
+// The FP32 kernels use FP32 copies of the nine components (A32, may be
+// absent).
 struct Area32 {
-  float* m[6];
+  float* m[9];
 };
 
 __global__ void area_kernel(Dims d, Met M, Met A, Area32 A32) {
@@ -114,7 +114,7 @@ __global__ void area_kernel(Dims d, Met M, Met A, Area32 A32) {
   A.m[9][o] = 1.0 / J;
   if (A32.m[0]) {
 #pragma unroll
-    for (int m = 0; m < 6; ++m) A32.m[m][o] = (float)A.m[m][o];
+    for (int m = 0; m < 9; ++m) A32.m[m][o] = (float)A.m[m][o];
   }
 }
 
@@ -188,6 +188,17 @@ __global__ void soa_to_aos(Dims d, const double* q, double* aos) {
   const long o = node_off(d, i, j, k);
 #pragma unroll
   for (int n = 0; n < NEQ; ++n) aos[5 * e + n] = q[n * d.VOL + o];
+}
+
+// the FP32 copies of a state, one per state buffer (two nodes per thread)
+__global__ void narrow_state(const double2* q, float2* a, float2* b, float2* c, long n) {
+  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const double2 v = q[e];
+  const float2 f = make_float2((float)v.x, (float)v.y);
+  a[e] = f;
+  b[e] = f;
+  c[e] = f;
 }
 
 // field over the N nodes -> dense IM*JM*KM
@@ -324,14 +335,14 @@ inline unsigned nb(long n) { return (unsigned)((n + 255) / 256); }
 }  // namespace
 
 cudaError_t launch_metrics(const Dims& d, const double* x, const double* y, const double* z, double* const met[10],
-                           double* const area[10], float* const area32[6], int wrap, cudaStream_t s) {
+                           double* const area[10], float* const area32[9], int wrap, cudaStream_t s) {
   Met M, A;
   Area32 A32;
   for (int m = 0; m < 10; ++m) {
     M.m[m] = met[m];
     A.m[m] = area[m];
   }
-  for (int m = 0; m < 6; ++m) A32.m[m] = area32 ? area32[m] : nullptr;
+  for (int m = 0; m < 9; ++m) A32.m[m] = area32 ? area32[m] : nullptr;
   metrics_nodes<<<nb((long)d.IM * d.JM * d.KM), 256, 0, s>>>(d, x, y, z, M);
   if (wrap > 0) metrics_wrap<<<nb(2L * wrap * d.JM * d.KM), 256, 0, s>>>(d, M, wrap);
   metrics_ghosts<<<nb((long)d.IG * d.JG * d.KG), 256, 0, s>>>(d, M);
@@ -374,6 +385,13 @@ cudaError_t launch_primitive(const Dims& d, const double* q, double* const prim[
 
 cudaError_t launch_aos_to_soa(const Dims& d, const double* aos, double* q, cudaStream_t s) {
   aos_to_soa<<<nb((long)d.IG * d.JG * d.KG), 256, 0, s>>>(d, aos, q);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_narrow_state(const Dims& d, const double* q, float* const q32[3], cudaStream_t s) {
+  const long n = NEQ * d.VOL / 2;  // VOL is a multiple of 32
+  narrow_state<<<nb(n), 256, 0, s>>>(reinterpret_cast<const double2*>(q), reinterpret_cast<float2*>(q32[0]),
+                                     reinterpret_cast<float2*>(q32[1]), reinterpret_cast<float2*>(q32[2]), n);
   return cudaGetLastError();
 }
 

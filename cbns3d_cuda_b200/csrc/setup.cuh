@@ -11,7 +11,7 @@ namespace cbns {
 // the nodes i < wrap and i >= IM - wrap take the metrics of the nodes
 // IM - 2*wrap away, before the ghost extension.
 cudaError_t launch_metrics(const Dims& d, const double* x, const double* y, const double* z, double* const met[10],
-                           double* const area[10], float* const area32[6], int wrap, cudaStream_t s);
+                           double* const area[10], float* const area32[9], int wrap, cudaStream_t s);
 cudaError_t launch_ic(const Dims& d, double* const prim[6], double angle_deg, double p_inf, int viscous,
                       cudaStream_t s);
 // Case initial states on the ghosted box (kind CBNS_CASE_*, prm as in
@@ -22,6 +22,8 @@ cudaError_t launch_conservative(const Dims& d, double* const prim[6], double* q,
 cudaError_t launch_primitive(const Dims& d, const double* q, double* const prim[6], double gam1, double gM2,
                              cudaStream_t s);
 cudaError_t launch_aos_to_soa(const Dims& d, const double* aos, double* q, cudaStream_t s);
+// the FP32 copies of state q (all three buffers hold q)
+cudaError_t launch_narrow_state(const Dims& d, const double* q, float* const q32[3], cudaStream_t s);
 cudaError_t launch_soa_to_aos(const Dims& d, const double* q, double* aos, cudaStream_t s);
 cudaError_t launch_gather_nodes(const Dims& d, const double* f, double* out, cudaStream_t s);
 cudaError_t launch_gather_ghosted(const Dims& d, const double* f, double* out, cudaStream_t s);

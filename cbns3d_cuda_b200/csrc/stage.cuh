@@ -7,25 +7,28 @@
 
 namespace cbns {
 
-// TMA tensor maps of the stage kernels' plane staging (tma.cuh), 4-D: x,
-// rows, planes, fields.  FP32 kernels: q_a the stage input's i-side halo box
-// (4 x 15 x 1 x 5, FP64), q_b its j-side halo box (16 x 3 x 1 x 5), xi / eta
-// the FP32 face-node area vectors (the 6 area32 components; 24 x 15 x 1 x 3
-// and 16 x 17 x 1 x 3).  FP64 TMA kernel: q_a the ring column box (16 x 15 x
-// 1 x 5), q_b the plane-with-halo box (24 x 21 x 1 x 5), xi / eta the FP64
-// area vectors (the 10 area components; the same boxes).
+// TMA tensor maps of the stage kernels (tma.cuh), 4-D: x, rows, planes,
+// fields.  q_a: the ring column box (16 x 15 x 1 x 5) of the stage input, q_b
+// its plane-with-halo box (24 x 21 x 1 x 5), xi / eta the face-node area
+// vectors (24 x 15 x 1 x 3 and 16 x 17 x 1 x 3), zeta (16 x 15 x 1 x 3): FP64 in
+// the FP64 kernel (the 10 area components), FP32 copies in the FP32 kernels
+// (the 9 area32 components).  The FP64 update operands' boxes (16 x 15 x 1 x 5,
+// iJ x 1), prefetched into L2: q0, qp, iJ, and in the FP32 kernels of viscous
+// runs dfv (FP32 elements, x 4).
 struct StageMaps {
-  CUtensorMap q_a, q_b, xi, eta;
+  CUtensorMap q_a, q_b, xi, eta, zeta, q0, qp, iJ, dfv;
 };
 
 struct StageArgs {
-  StageMaps tm;        // FP32 kernels: TMA maps for src and area32
+  StageMaps tm;        // TMA maps, first: the batched kernels copy what follows
   Dims d;
   double gamma, gam1, gam1_inv, gM2;
   const double* src;   // stage input (stencil source), 5 fields
   const double* q0;    // the reference's Q at the node (RK base)
   const double* qp;    // the reference's Q_p at the node (stages 2, 3)
   double* out;         // stage output (5 fields), or the dense RHS array in mode 0
+  float* out32;        // FP32 kernels: the FP32 copy of the stage output
+  const float* src32;  // FP32 kernels: the FP32 copy of the stage input
   const double* met[10];
   const double* area[10];  // J*grad(xi|eta|zeta) per node, then 1/J
   const double* dfv[4];    // viscous: the divergence of the node fluxes (visc.cu; FP32 elements in the FP32 kernels)
@@ -33,12 +36,21 @@ struct StageArgs {
   StepState* st;       // dt, done flag, spectral-radius max
   const unsigned char* mask;  // hybrid: per-face sensor decision (null: plain flux everywhere)
   float* wflux;        // hybrid: WENO5 flux of each WENO5 face (8 floats per face, 5 used)
-  const float* area32[6];  // FP32 kernels: J*grad(xi), J*grad(eta) per node in FP32
+  const float* area32[9];  // FP32 kernels: J*grad(xi), J*grad(eta), J*grad(zeta) per node in FP32
   int q0_is_src, qp_is_src;  // RK operands that equal the stage input (read from the ring)
   int ntile_i, ntile_j, kchunk;
   int visdiv;          // CBNS_VISDIV_*
   int sigma;           // accumulate the interior spectral-radius max (inviscid stage 3)
 };
+
+// StageArgs of a batch item from the device table into shared memory, without
+// the tensor maps (read where they lie); nt threads.
+__device__ __forceinline__ void copy_args(StageArgs* to, const StageArgs* from, int nt) {
+  const int* src = reinterpret_cast<const int*>(from);
+  int* dst = reinterpret_cast<int*>(to);
+  for (int e = (int)(sizeof(StageMaps) / sizeof(int)) + threadIdx.x; e < (int)(sizeof(StageArgs) / sizeof(int)); e += nt)
+    dst[e] = __ldg(src + e);
+}
 
 // Many blocks in one launch (a persistent work queue): args[b] are the
 // StageArgs of block b, its work items (tile, k chunk) are numbered
@@ -55,6 +67,10 @@ struct BatchStage {
 // variant: a compiled occupancy variant, 0 .. stage_variants(fp32)-1.
 cudaError_t launch_stage(const StageArgs& a, int mode, bool visc, bool fp32, int variant, cudaStream_t s);
 int stage_variants(bool fp32, bool hybrid);
+// The FP32 kernels (stage32.cu); variant 0: registers for 2 CTAs per SM, else 3.
+void stage32_prepare();
+cudaError_t launch_stage32(const StageArgs& a, int mode, bool visc, int variant, cudaStream_t s);
+cudaError_t launch_stage32_batched(const BatchStage& b, int mode, bool visc, bool hybrid, cudaStream_t s);
 // Hybrid: list the faces whose decision byte is set (once per step, after the
 // decisions are final; each face kind in its own list, st->weno_listed[kind]
 // receiving its length) ...

@@ -75,6 +75,14 @@ __device__ __forceinline__ void load_4d(void* dst, const CUtensorMap* map, int x
       : "memory");
 }
 
+// the same box's lines into L2
+__device__ __forceinline__ void prefetch_4d(const CUtensorMap* map, int x, int y, int z, int f) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(
+                   reinterpret_cast<unsigned long long>(map)),
+               "r"(x), "r"(y), "r"(z), "r"(f)
+               : "memory");
+}
+
 }  // namespace tma
 
 // Host: encode a 4-D tiled tensor map over `fields` node arrays of element

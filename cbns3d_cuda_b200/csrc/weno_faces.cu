@@ -14,10 +14,9 @@
 // rejected the step's decisions, or the sensor timed out) the pass evaluates
 // every face.
 //
-// Stencils are read from the stage input in FP64 and rounded to FP32 as the
-// stage kernel rounds its staged copies, and the face normals are formed from
-// the same FP32 area vectors, so a face gets the flux the stage kernel would
-// compute for it.
+// Stencils are read from the stage input's FP32 copy, as the stage kernel reads
+// them, and the face normals are formed from the same FP32 area vectors, so a
+// face gets the flux the stage kernel would compute for it.
 #include "cbns_common.cuh"
 #include "face_flux.cuh"
 #include "sensor_kernels.cuh"
@@ -30,7 +29,7 @@ namespace {
 constexpr int LT = 256;       // list kernel: threads
 constexpr int LB = 16;        // decision bytes per thread (one 16-byte load)
 constexpr int LCH = LT * LB;  // faces per CTA
-constexpr int WT = 256;       // evaluation kernel: threads
+constexpr int WT = 128;       // evaluation kernel: threads
 
 // A list entry: the face index and, packed, its kind (0 i-, 1 j-, 2 k-face,
 // bits 30-31) and the node offset of its low node (bits 0-29; contexts of the
@@ -204,81 +203,80 @@ __global__ void __launch_bounds__(LT) weno_list_batched(const ListArgs* args, co
   list_body(a.d, a.mask, a.nf, a.st, a.list, a.check_done, a.every, blockIdx.x - (unsigned)__ldg(cta + b));
 }
 
-// The WENO5 flux of one face of a's stage input into a.wflux: face w of the
-// list (or, with all set, face w of the block).  Each thread stages its face's
-// stencil in FP32 in its own column of shared memory (my, stride WT), so the
-// flux reads it there instead of keeping it in registers.
-__device__ __forceinline__ void weno_face(const StageArgs& a, bool all, long w, const int2* list, float* my) {
-  const Dims& d = a.d;
-  const long VOL = d.VOL;
+// A face of a's stage input: its index, low node and kind, from entry w of the
+// list or (with all set) face w of the block.
+struct FaceRef {
   long e, oa;
   int kind;
+};
+__device__ __forceinline__ FaceRef face_ref(const Dims& d, bool all, long w, const int2* list) {
   if (all) {
     const long nfi = (long)(d.IM - 1) * (d.JM - 2) * (d.KM - 2);
     const long nfj = (long)(d.IM - 2) * (d.JM - 1) * (d.KM - 2);
     FaceCursor c;
     cursor_set(d, nfi, nfj, w, c);
-    e = w;
-    kind = c.kind;
-    oa = c.oa;
-  } else {
-    const int2 le = __ldg(list + w);
-    e = le.x;
-    kind = (int)((unsigned)le.y >> 30);
-    oa = (long)((unsigned)le.y & 0x3fffffffu);
+    return FaceRef{w, c.oa, c.kind};
   }
-  long o0, s;  // first stencil node and the stride along the face normal
-  float nx, ny, nz;
-  if (kind == 0) {
-    // i-face between node oa and the next along i
-    o0 = oa - 2;
-    s = 1;
-    nx = 0.5f * (__ldg(a.area32[0] + oa) + __ldg(a.area32[0] + oa + 1));
-    ny = 0.5f * (__ldg(a.area32[1] + oa) + __ldg(a.area32[1] + oa + 1));
-    nz = 0.5f * (__ldg(a.area32[2] + oa) + __ldg(a.area32[2] + oa + 1));
-  } else if (kind == 1) {
-    // j-face between node oa and the next along j
-    o0 = oa - 2 * d.PX;
-    s = d.PX;
-    nx = 0.5f * (__ldg(a.area32[3] + oa) + __ldg(a.area32[3] + oa + d.PX));
-    ny = 0.5f * (__ldg(a.area32[4] + oa) + __ldg(a.area32[4] + oa + d.PX));
-    nz = 0.5f * (__ldg(a.area32[5] + oa) + __ldg(a.area32[5] + oa + d.PX));
-  } else {
-    // k-face between node oa and the next along k
-    o0 = oa - 2 * d.PL;
-    s = d.PL;
-    nx = 0.5f * ((float)__ldg(a.area[6] + oa) + (float)__ldg(a.area[6] + oa + d.PL));
-    ny = 0.5f * ((float)__ldg(a.area[7] + oa) + (float)__ldg(a.area[7] + oa + d.PL));
-    nz = 0.5f * ((float)__ldg(a.area[8] + oa) + (float)__ldg(a.area[8] + oa + d.PL));
-  }
-  // the stencil in FP32: all 30 loads in flight at once, each value converted once
+  const int2 le = __ldg(list + w);
+  return FaceRef{le.x, (long)((unsigned)le.y & 0x3fffffffu), (int)((unsigned)le.y >> 30)};
+}
+
+// The WENO5 fluxes of the two faces w0 and w1 (the same kind) into a.wflux.
+// Each thread stages its pair's stencil values in its own column of shared
+// memory (my, stride WT), so the packed flux reads them there, pairs in one
+// load, instead of keeping them in registers.
+__device__ __forceinline__ void weno_pair(const StageArgs& a, bool all, long w0, long w1, const int2* list, float2* my) {
+  const Dims& d = a.d;
+  const FaceRef r0 = face_ref(d, all, w0, list), r1 = face_ref(d, all, w1, list);
+  // along the face normal: the stride s; area vector components 3*kind ..
+  const long s = r0.kind == 0 ? 1 : r0.kind == 1 ? d.PX : d.PL;
   {
-    const double* sp = a.src + o0;
+    const float *p0 = a.src32 + r0.oa - 2 * s, *p1 = a.src32 + r1.oa - 2 * s;
 #pragma unroll
     for (int q = 0; q < NEQ; ++q)
 #pragma unroll
-      for (int p = 0; p < 6; ++p) my[(q * 6 + p) * WT] = (float)__ldg(sp + q * VOL + p * s);
+      for (int p = 0; p < 6; ++p)
+        my[(q * 6 + p) * WT] = make_float2(__ldg(p0 + q * d.VOL + p * s), __ldg(p1 + q * d.VOL + p * s));
   }
-  auto ld = [&](int p, int q) -> float { return my[(q * 6 + p) * WT]; };
+  F2 n[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const float* ar = a.area32[0] + (3 * r0.kind + m) * d.VOL;
+    n[m] = mk(0.5f * (__ldg(ar + r0.oa) + __ldg(ar + r0.oa + s)), 0.5f * (__ldg(ar + r1.oa) + __ldg(ar + r1.oa + s)));
+  }
+  auto ld = [&](int p, int q) -> F2 {
+    const float2 v = my[(q * 6 + p) * WT];
+    return mk(v.x, v.y);
+  };
   const FluxConsts<float> C{(float)a.gamma, (float)a.gam1, (float)a.gam1_inv};
-  float f[5];
-  face_flux<float>(ld, nx, ny, nz, C, f);
-  float* out = a.wflux + 8 * e;
-  *reinterpret_cast<float4*>(out) = make_float4(f[0], f[1], f[2], f[3]);
-  out[4] = f[4];
+  F2 f[5];
+  face_flux<F2>(ld, n[0], n[1], n[2], C, f);
+  float x[5], y[5];
+#pragma unroll
+  for (int m = 0; m < NEQ; ++m) halves(f[m], x[m], y[m]);
+  auto put = [&](long e, const float* v) {
+    float* out = a.wflux + 8 * e;
+    *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+    out[4] = v[4];
+  };
+  put(r0.e, x);
+  put(r1.e, y);
 }
 
-// One thread per listed face, or per face while force_weno is set.  The CTAs
-// are shared out among the three kinds' lists in proportion to their lengths
-// (at least one for a kind with faces), and each kind's CTAs walk its list
+// Two listed faces per thread (faces while force_weno is set), WT apart in the
+// list so that neighbouring threads read neighbouring faces.  The CTAs are
+// shared out among the three kinds' lists in proportion to their lengths (at
+// least one for a kind with faces), and each kind's CTAs walk its list
 // grid-stride, so the three kinds advance through the grid's planes side by
-// side and the stencils they share stay in L2.  Built for 3 CTAs per SM (80
-// registers): the faces' stencil loads are the wait, and 24 warps per SM hide
-// more of it than 16 (10% faster on the bench grid); the staged stencils take
-// 30 KB of shared memory per CTA.
+// side and the stencils they share stay in L2.  A list of odd length ends with
+// its last face evaluated twice by one thread.
+// Bound by the stencil loads (24% of issue slots idle on them) and the FP32
+// pipe.  Built for 3 CTAs of 128 threads per SM (168 registers).  One launch of
+// a 256x256x128 hybrid step: 171 us with one face per thread from the FP64
+// state (256 threads, 80 registers), 149 us in pairs from its FP32 copy.
 __global__ void __launch_bounds__(WT, 3) weno_faces_kernel(const __grid_constant__ StageArgs a, int mode, long nf,
                                                            const int2* list) {
-  __shared__ float stn[NEQ * 6][WT];
+  __shared__ float2 stn[NEQ * 6][WT];
   const StepState* st = a.st;
   if (mode != 0 && st->done) return;
   const bool all = st->force_weno != 0;
@@ -298,8 +296,8 @@ __global__ void __launch_bounds__(WT, 3) weno_faces_kernel(const __grid_constant
   const int k = c < b1 ? 0 : (c < b2 ? 1 : 2);
   const int base = k == 0 ? 0 : (k == 1 ? b1 : b2);
   const int g = k == 0 ? b1 : (k == 1 ? b2 - b1 : G - b2);
-  for (long w = (long)(c - base) * WT + threadIdx.x; w < len[k]; w += (long)g * WT)
-    weno_face(a, all, first[k] + w, list, &stn[0][threadIdx.x]);
+  for (long w = (long)(c - base) * 2 * WT + threadIdx.x; w < len[k]; w += (long)g * 2 * WT)
+    weno_pair(a, all, first[k] + w, first[k] + min(w + WT, len[k] - 1), list, &stn[0][threadIdx.x]);
 }
 
 int g_weno_grid = 0;  // persistent grid of the evaluation kernel: resident CTAs of the device
