@@ -30,6 +30,7 @@
 // vectors and 1/J (80 B), the RK base (0-40 B) and the output (40 B).
 #include "cbns_common.cuh"
 #include "face_flux.cuh"
+#include "sigma.cuh"
 #include "stage.cuh"
 #include "tma.cuh"
 
@@ -52,6 +53,14 @@ static_assert(NFI == 7 * 32 + 16 + TJ, "face mapping of the face rounds");
 constexpr int NSX = (TI + 2) * TJ;  // i-face nodes (i0-1 .. i0+16)
 constexpr int NSY = TI * (TJ + 2);  // j-face nodes (j0-1 .. j0+15)
 constexpr int NHI = 2 * H * TJ, NHJ = 2 * H * TI;  // halo nodes of a plane: i-halo, j-halo
+
+// x / 3: the product with the rounded 1/3 corrected by its exact residual,
+// three operations for the division's dozen (the residual x - 3q is exact, so
+// the result is x/3 rounded once more).
+__device__ __forceinline__ double third(double x) {
+  const double q = ml(x, 1.0 / 3.0);
+  return fm(fm(-3.0, q, x), 1.0 / 3.0, q);
+}
 
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
@@ -285,6 +294,9 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const StageMaps* 
 
   double smax = 0.0;  // running spectral-radius max (stage 3, inviscid)
   bool snan = false;
+  constexpr bool kSigma = MODE == 3 && !VISC;
+  __shared__ int best;  // the largest spectral radius met so far (sigma.cuh)
+  if (kSigma && a.sigma && t == 32) best = __float_as_int(sigma_start(st));
 
   for (int k = kb; k < ke; ++k) {
     if (t == 0 && k + 1 < ke) prefetch_set(k + 1);
@@ -393,6 +405,17 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const StageMaps* 
     }
     // round C: the k+1/2 face of this column
     if (col_valid) k_face(k, za, zb, fkp);
+    // stage 3's spectral radius: the column's area vectors in FP32 for its
+    // bound, before the staging is refilled
+    float ar[9];
+    if (kSigma && col_valid) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        ar[m] = (float)ax(m, cy, cx + 1);
+        ar[3 + m] = (float)ay(m, cy + 1, cx);
+        ar[6 + m] = (float)za[m];
+      }
+    }
     __syncthreads();
     // TMA kernel: plane k+1's set travels during the update (it
     // overwrites the plane, the area vectors and plane k-2's ring slot, which
@@ -414,70 +437,49 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const StageMaps* 
       if (MODE == 0) {
         const long r = 5L * ((ci - 1) + (long)(d.IM - 2) * ((cj - 1) + (long)(d.JM - 2) * (k - 1)));
 #pragma unroll
-        for (int n = 0; n < NEQ; ++n) a.out[r + n] = df[n] * iJ;
+        for (int n = 0; n < NEQ; ++n) a.out[r + n] = ml(df[n], iJ);
       } else {
         const int sk = k % 6;
         double q[NEQ];
 #pragma unroll
         for (int n = 0; n < NEQ; ++n) {
-          const double L = dt * (df[n] * iJ);
+          // explicit roundings: the variants and the batched form agree to the bit
+          const double x = ml(df[n], iJ);
           const long e = n * VOL + o;
           const double qin = sm.ring[sk][n][t];
           const double q0v = MODE == 3 ? a.q0[e] : __ldg(a.q0 + e);
           const double qpv = MODE >= 2 ? __ldg(a.qp + e) : 0.0;
-          if (MODE == 1) {
-            q[n] = (a.q0_is_src ? qin : q0v) - L;
-          } else if (MODE == 2) {
-            q[n] = 0.75 * q0v + 0.25 * ((a.qp_is_src ? qin : qpv) - L);
-          } else {
-            q[n] = (q0v + 2.0 * ((a.qp_is_src ? qin : qpv) - L)) / 3.0;
-          }
+          if (MODE == 1) q[n] = fm(-dt, x, a.q0_is_src ? qin : q0v);
+          else if (MODE == 2) q[n] = fm(0.25, fm(-dt, x, a.qp_is_src ? qin : qpv), ml(0.75, q0v));
+          else q[n] = third(fm(2.0, fm(-dt, x, a.qp_is_src ? qin : qpv), q0v));
         }
 #pragma unroll
         for (int n = 0; n < NEQ; ++n) a.out[n * VOL + o] = q[n];
-        if (VISC || a.sigma) {
+        if (VISC) {
           const double r = q[0], ir = rcp_(r);
           const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
           const double ke = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
           const double pp = __dmul_rn(a.gam1, __fma_rn(-__dmul_rn(0.5, r), ke, q[4]));
-          if (VISC) {
-            a.prim[0][o] = r;
-            a.prim[1][o] = uu;
-            a.prim[2][o] = vv;
-            a.prim[3][o] = ww;
-            a.prim[4][o] = pp;
-            a.prim[5][o] = a.gM2 * pp / r;
-          } else {
-            // grad(xi), grad(eta), grad(zeta) = area vectors / J: xi and eta
-            // from the plane's staged face-node area vectors, from memory in
-            // the TMA kernel (its staging is being refilled); zeta from the
-            // registers
-            double g[9];
+          a.prim[0][o] = r;
+          a.prim[1][o] = uu;
+          a.prim[2][o] = vv;
+          a.prim[3][o] = ww;
+          a.prim[4][o] = pp;
+          a.prim[5][o] = a.gM2 * pp / r;
+        } else if (kSigma && a.sigma) {
+          // in FP64 only where the FP32 bound reaches the largest met so far
+          float qf[NEQ], small;
 #pragma unroll
-            for (int m = 0; m < 3; ++m) {
-              if constexpr (TMA) {
-                g[m] = __ldg(a.area[m] + o);
-                g[3 + m] = __ldg(a.area[3 + m] + o);
-              } else {
-                g[m] = ax(m, cy, cx + 1);
-                g[3 + m] = ay(m, cy + 1, cx);
-              }
-              g[6 + m] = za[m];
-            }
-            // explicit roundings: every compilation of this kernel (single
-            // and batched) then gives the same dt to the last bit
-            const double cs = sqrt_(__dmul_rn(__dmul_rn(a.gamma, pp), ir));
-            double s = 0.0;
+          for (int n = 0; n < NEQ; ++n) qf[n] = (float)q[n];
+          const float b = sigma_bound(qf, ar, (float)iJ, (float)a.gamma, (float)a.gam1, small);
+          if (sigma_reaches(b, small, __int_as_float(*(volatile int*)&best))) {
+            double A[9];
 #pragma unroll
-            for (int dd = 0; dd < 3; ++dd) {
-              const double mx = g[3 * dd], my = g[3 * dd + 1], mz = g[3 * dd + 2];
-              const double un = __fma_rn(ww, mz, __fma_rn(vv, my, __dmul_rn(uu, mx)));
-              const double nn = __fma_rn(mz, mz, __fma_rn(my, my, __dmul_rn(mx, mx)));
-              s = __dadd_rn(s, __fma_rn(cs, sqrt_(nn), fabs(un)));
-            }
-            s = __dmul_rn(s, iJ);
+            for (int m = 0; m < 9; ++m) A[m] = __ldg(a.area[m] + o);
+            const double s = sigma_exact(q, A, iJ, a.gamma, a.gam1);
             if (s != s) snan = true;
             smax = fmax(smax, s);
+            sigma_found(&best, s);
           }
         }
       }
@@ -497,7 +499,7 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const StageMaps* 
       tma::bar_inval(&t64->bar[1]);
     }
   }
-  if (MODE != 0 && !VISC && a.sigma) {
+  if (kSigma && a.sigma) {
     // CTA max, one atomic per CTA
     __shared__ double red[NT / 32];
     __shared__ int rnan;

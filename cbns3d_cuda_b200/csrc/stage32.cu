@@ -46,6 +46,7 @@
 // fluxes of plane k are asked into L1 at its start.
 #include "cbns_common.cuh"
 #include "face_flux.cuh"
+#include "sigma.cuh"
 #include "stage.cuh"
 #include "tma.cuh"
 
@@ -70,6 +71,7 @@ struct alignas(128) Smem32 {
   float fi[2][NEQ][TJ][TI + 1];            // plane p in buffer p & 1
   float fj[2][NEQ][TJ + 1][TI];
   alignas(8) unsigned long long bar[2];
+  int best;  // the largest spectral radius met so far (sigma.cuh)
 };
 constexpr size_t kSmem = sizeof(Smem32) + 128;
 // transaction bytes: a plane's set, the warm-up set (six ring planes, two zeta planes)
@@ -123,6 +125,8 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
     }
   };
 
+  constexpr bool kSigma = MODE == 3 && !VISC;
+  if (kSigma && a.sigma && t == 32) sm.best = __float_as_int(sigma_start(st));
   if (t == 0) {
     tma::bar_init(&sm.bar[0]);
     tma::bar_init(&sm.bar[1]);
@@ -322,7 +326,7 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
     // it; with the WENO5 flux each column's in its update (loaded ahead they
     // spill)
     const long o0 = node_off(d, ci, cj0, k), o1 = node_off(d, ci, cj1, k);
-    double iJ[2], q0v[2][NEQ], qpv[2][NEQ], zeta[2][3];
+    double iJ[2] = {0.0, 0.0}, q0v[2][NEQ], qpv[2][NEQ];
     auto load_operands = [&](int q2) {
       if (!(q2 ? vC1 : vC0)) return;
       const long o = q2 ? o1 : o0;
@@ -333,10 +337,6 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
         q0v[q2][n] = MODE == 3 ? a.q0[n * VOL + o] : __ldg(a.q0 + n * VOL + o);
         if (MODE >= 2) qpv[q2][n] = __ldg(a.qp + n * VOL + o);
       }
-      if (MODE == 3 && !VISC) {
-#pragma unroll
-        for (int m = 0; m < 3; ++m) zeta[q2][m] = __ldg(a.area[6 + m] + o);
-      }
     };
     if (HYB) {
       load_operands(0);
@@ -345,18 +345,16 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
     // round C: the k+1/2 faces of the thread's columns
     F2 fkp[5];
     k_face(k, (mcur >> 4) & 3u, fkp);
-    // stage 3's spectral radius takes the plane's area vectors, whose buffers
-    // are refilled during the update
-    float gx[2][6];
-    if (MODE == 3 && !VISC && a.sigma) {
+    // stage 3's spectral radius: the columns' area vectors, whose buffers are
+    // refilled during the update
+    F2 ar[9];
+    if (kSigma) {
+      const int y1 = min(cy1, TJ - 1);
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        gx[0][m] = sm.xi[m][cy0][c + 4];
-        gx[0][3 + m] = sm.eta[m][cy0 + 1][c];
-        if (cy1 < TJ) {
-          gx[1][m] = sm.xi[m][cy1][c + 4];
-          gx[1][3 + m] = sm.eta[m][cy1 + 1][c];
-        }
+        ar[m] = mk(sm.xi[m][cy0][c + 4], sm.xi[m][y1][c + 4]);
+        ar[3 + m] = mk(sm.eta[m][cy0 + 1][c], sm.eta[m][y1 + 1][c]);
+        ar[6 + m] = mk(sm.zt[k & 1][m * NC + t], sm.zt[k & 1][m * NC + y1 * TI + c]);
       }
     }
     if (__syncthreads_or(!landed)) {
@@ -376,6 +374,7 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
       issue_ring_zeta(k + 1, nb);
     }
     // the update of the two columns
+    float qf[2][NEQ] = {{1.f, 0.f, 0.f, 0.f, 0.f}, {1.f, 0.f, 0.f, 0.f, 0.f}};
     float fk[2][5];
 #pragma unroll
     for (int n = 0; n < NEQ; ++n) halves(sb(fkp[n], fkm[n]), fk[0][n], fk[1][n]);
@@ -411,47 +410,50 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
 #pragma unroll
         for (int n = 0; n < NEQ; ++n) {
           a.out[n * VOL + o] = q[n];
-          a.out32[n * VOL + o] = (float)q[n];
+          a.out32[n * VOL + o] = qf[q2][n] = (float)q[n];
         }
-        if (VISC || (MODE == 3 && a.sigma)) {
+        if (VISC) {
           const double r = q[0], ir = rcp_(r);
           const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
           const double kk = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
           const double pp = __dmul_rn(a.gam1, __fma_rn(-__dmul_rn(0.5, r), kk, q[4]));
-          if (VISC) {
-            a.prim[0][o] = r;
-            a.prim[1][o] = uu;
-            a.prim[2][o] = vv;
-            a.prim[3][o] = ww;
-            a.prim[4][o] = pp;
-            a.prim[5][o] = a.gM2 * pp / r;
-          } else {
-            // grad(xi), grad(eta), grad(zeta) = area vectors / J, the spectral
-            // radius in FP64 from the FP32 copies of the xi and eta vectors
-            // (as the fluxes use them; dt moves by ~1e-7 relative) and the
-            // FP64 zeta vectors; explicit roundings, so every compilation of
-            // this kernel gives the same dt
-            double g[9];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-              g[m] = (double)gx[q2][m];
-              g[3 + m] = (double)gx[q2][3 + m];
-              g[6 + m] = zeta[q2][m];
-            }
-            const double cs = sqrt_(__dmul_rn(__dmul_rn(a.gamma, pp), ir));
-            double s = 0.0;
-#pragma unroll
-            for (int dd = 0; dd < 3; ++dd) {
-              const double mx = g[3 * dd], my = g[3 * dd + 1], mz = g[3 * dd + 2];
-              const double un = __fma_rn(ww, mz, __fma_rn(vv, my, __dmul_rn(uu, mx)));
-              const double nn = __fma_rn(mz, mz, __fma_rn(my, my, __dmul_rn(mx, mx)));
-              s = __dadd_rn(s, __fma_rn(cs, sqrt_(nn), fabs(un)));
-            }
-            s = __dmul_rn(s, iJ[q2]);
-            if (s != s) snan = true;
-            smax = fmax(smax, s);
-          }
+          a.prim[0][o] = r;
+          a.prim[1][o] = uu;
+          a.prim[2][o] = vv;
+          a.prim[3][o] = ww;
+          a.prim[4][o] = pp;
+          a.prim[5][o] = a.gM2 * pp / r;
         }
+      }
+    }
+    // stage 3: the columns whose FP32 bound reaches the largest spectral radius
+    // met so far are evaluated in FP64, from the FP32 copies of the xi and eta
+    // vectors (as the fluxes use them; dt moves by ~1e-7 relative) and the FP64
+    // zeta vectors
+    if (kSigma && a.sigma) {
+      F2 qb[NEQ], small;
+#pragma unroll
+      for (int n = 0; n < NEQ; ++n) qb[n] = mk(qf[0][n], qf[1][n]);
+      float b[2], sl[2];
+      const F2 bound = sigma_bound(qb, ar, mk((float)iJ[0], (float)iJ[1]), C.gamma, C.gam1, small);
+      halves(bound, b[0], b[1]);
+      halves(small, sl[0], sl[1]);
+      const float found = __int_as_float(*(volatile int*)&sm.best);
+#pragma unroll 1
+      for (int q2 = 0; q2 < 2; ++q2) {
+        if (!(q2 ? vC1 : vC0) || !sigma_reaches(q2 ? b[1] : b[0], q2 ? sl[1] : sl[0], found)) continue;
+        const long o = q2 ? o1 : o0;
+        double q[NEQ], A[9];
+#pragma unroll
+        for (int n = 0; n < NEQ; ++n) q[n] = a.out[n * VOL + o];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) A[m] = (double)__ldg(a.area32[m] + o);
+#pragma unroll
+        for (int m = 6; m < 9; ++m) A[m] = __ldg(a.area[m] + o);
+        const double s = sigma_exact(q, A, __ldg(a.area[9] + o), a.gamma, a.gam1);
+        if (s != s) snan = true;
+        smax = fmax(smax, s);
+        sigma_found(&sm.best, s);
       }
     }
 #pragma unroll
@@ -465,7 +467,7 @@ __device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps
     tma::bar_inval(&sm.bar[0]);
     tma::bar_inval(&sm.bar[1]);
   }
-  if (MODE == 3 && !VISC && a.sigma) {
+  if (kSigma && a.sigma) {
     // CTA max, one atomic per CTA
     __shared__ double red[NT / 32];
     __shared__ int rnan;
