@@ -750,13 +750,15 @@ int batch_sensor_tables(cbns_batch* b) {
   return CBNS_OK;
 }
 
+// k planes per work item of a batch's stage launches.  Stage 2 at 4 / 6 / 8 / 12
+// / 16 / 24 planes: 12 FP64 blocks (2.2 M nodes) 575 / 582 / 589 / 615 / 604 /
+// 672 us, 64 viscous hybrid blocks (10.8 M) 959 / 943 / 943 / 946 / 951 / 981:
+// longer items leave slots idle at the end of a small batch, shorter ones start
+// more often.
+constexpr int kBatchKChunk = 8;
+
 // The StageArgs of the three stages of every block for the fixed buffer roles
 // P0 = Q, P1 = spare, P2 = Q_p (as enqueue_step), uploaded to the device.
-// k planes per work item of a batch's stage launches: measured on the
-// 64-block workload (16 planes: 11.31 ms per step, 32: 11.33, whole columns:
-// 11.66, the blocks' own chunks of about 9 planes: 11.54)
-constexpr int kBatchKChunk = 16;
-
 int batch_tables(cbns_batch* b) {
   const int nb = (int)b->blk.size();
   std::vector<StageArgs> tab(3 * nb);
@@ -770,9 +772,8 @@ int batch_tables(cbns_batch* b) {
     tab[0 * nb + i] = stage_args(c, P0, P0, P0, P1, false);
     tab[1 * nb + i] = stage_args(c, P1, P0, P1, P2, false);
     tab[2 * nb + i] = stage_args(c, P2, P0, P2, P0, !b->visc);
-    // the batch's own chunking: its work queue balances the blocks' items, so
-    // chunks of up to kBatchKChunk planes instead of each block's (sized for
-    // the block alone on the whole GPU)
+    // the batch's own chunking instead of each block's (sized for the block
+    // alone on the whole GPU)
     const int kc = std::min(c->d.KM - 2, kBatchKChunk);
     for (int r = 0; r < 3; ++r) tab[r * nb + i].kchunk = kc;
     start[i + 1] = start[i] + c->ntile_i * c->ntile_j * ((c->d.KM - 2 + kc - 1) / kc);

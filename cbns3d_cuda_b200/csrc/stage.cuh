@@ -19,8 +19,7 @@ struct StageMaps {
   CUtensorMap q_a, q_b, xi, eta, zeta, q0, qp, iJ, dfv;
 };
 
-struct StageArgs {
-  StageMaps tm;        // TMA maps, first: the batched kernels copy what follows
+struct StageCore {
   Dims d;
   double gamma, gam1, gam1_inv, gM2;
   const double* src;   // stage input (stencil source), 5 fields
@@ -42,14 +41,16 @@ struct StageArgs {
   int visdiv;          // CBNS_VISDIV_*
   int sigma;           // accumulate the interior spectral-radius max (inviscid stage 3)
 };
+struct StageArgs : StageCore {
+  StageMaps tm;
+};
 
-// StageArgs of a batch item from the device table into shared memory, without
-// the tensor maps (read where they lie); nt threads.
-__device__ __forceinline__ void copy_args(StageArgs* to, const StageArgs* from, int nt) {
+// A batch item's StageCore from the device table into shared memory (its tensor
+// maps are read where they lie); nt threads.
+__device__ __forceinline__ void copy_core(StageCore* to, const StageCore* from, int nt) {
   const int* src = reinterpret_cast<const int*>(from);
   int* dst = reinterpret_cast<int*>(to);
-  for (int e = (int)(sizeof(StageMaps) / sizeof(int)) + threadIdx.x; e < (int)(sizeof(StageArgs) / sizeof(int)); e += nt)
-    dst[e] = __ldg(src + e);
+  for (int e = threadIdx.x; e < (int)(sizeof(StageCore) / sizeof(int)); e += nt) dst[e] = __ldg(src + e);
 }
 
 // Many blocks in one launch (a persistent work queue): args[b] are the

@@ -82,7 +82,7 @@ __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefe
 
 // The work of one CTA: tile `tile` of the block's (i, j) tiling, k chunk `kc`.
 template <bool VISC, int MODE, bool HYB>
-__device__ __forceinline__ void stage32_body(const StageArgs& a, const StageMaps* tm, int tile, int kc,
+__device__ __forceinline__ void stage32_body(const StageCore& a, const StageMaps* tm, int tile, int kc,
                                              unsigned char* smem_raw) {
   Smem32& sm = *reinterpret_cast<Smem32*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const StepState* st = a.st;
@@ -496,16 +496,15 @@ __global__ void __launch_bounds__(NT, NB) stage32_kernel(const __grid_constant__
 template <bool VISC, int MODE, bool HYB>
 __global__ void __launch_bounds__(NT, 3) stage32_kernel_batched(const BatchStage b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ StageArgs args;
+  __shared__ StageCore args;
   __shared__ int item;
   for (;;) {
     if (threadIdx.x == 0) item = (int)atomicAdd(b.counter, 1u);
     __syncthreads();
     const int w = item;
     if (w >= b.total) break;
-    int blk = 0;
-    while (blk + 1 < b.nblocks && __ldg(b.start + blk + 1) <= w) ++blk;
-    copy_args(&args, b.args + blk, NT);
+    const int blk = block_of_cta(b.start, b.nblocks, w);
+    copy_core(&args, b.args + blk, NT);
     __syncthreads();
     const int local = w - __ldg(b.start + blk);
     const int ntiles = args.ntile_i * args.ntile_j;
