@@ -18,8 +18,8 @@
 // every face), only their primitives and spectral radii are formed; with
 // CBNS_BC_CHARACTERISTIC three launches (i, j, k faces) first set every
 // boundary node and its ghosts to a characteristic far-field state.  With
-// CBNS_BC_OGRID: phase 2 with the wall on every i, the characteristic state on
-// j = JM-1, phase 3, then the copies across the periodic seam in i.
+// CBNS_BC_OGRID (bc_ogrid): phase 2 with the wall on every i, the characteristic
+// state on j = JM-1, phase 3, and the copies across the periodic seam in i.
 // The reference runs these as __syncthreads-separated phases of one kernel, so
 // its cross-CTA reads (wake mirror, k-face copies of j-face results) are races;
 // separate launches give the program-order result, which is what the reference
@@ -48,6 +48,16 @@ __device__ __forceinline__ PrimV prim_of(const double* q, long o, long VOL, doub
   s.v = q[2 * VOL + o] / s.r;
   s.w = q[3 * VOL + o] / s.r;
   s.p = gam1 * (q[4 * VOL + o] - 0.5 * s.r * (s.u * s.u + s.v * s.v + s.w * s.w));
+  return s;
+}
+
+__device__ __forceinline__ PrimV prim_of(const double q[NEQ], double gam1) {
+  PrimV s;
+  s.r = q[0];
+  s.u = q[1] / s.r;
+  s.v = q[2] / s.r;
+  s.w = q[3] / s.r;
+  s.p = gam1 * (q[4] - 0.5 * s.r * (s.u * s.u + s.v * s.v + s.w * s.w));
   return s;
 }
 
@@ -123,6 +133,65 @@ __global__ void bc_phase1(const BCArgs a) {
   }
 }
 
+// The wall at (i, 0, k) from the interior nodes above it: the state of j = 0 (w[0])
+// and of its ghosts j = -1, -2 (w[1], w[2]).
+__device__ __forceinline__ void wall_column(const BCArgs& a, int i, int k, double w[NG + 1][NEQ]) {
+  const Dims& d = a.d;
+  const long VOL = d.VOL;
+  const double gam1 = a.gam1;
+  double q[NG + 1][NEQ];
+#pragma unroll
+  for (int l = 1; l <= NG; ++l)
+#pragma unroll
+    for (int c = 0; c < NEQ; ++c) q[l][c] = a.q[c * VOL + node_off(d, i, l, k)];
+  if (a.viscous) {
+    // adiabatic no-slip wall
+    const double rr = q[1][0], ru = q[1][1], rv = q[1][2], rw = q[1][3];
+    const double pp = gam1 * (q[1][4] - 0.5 * (ru * ru + rv * rv + rw * rw) / rr);
+    w[0][0] = rr;
+    w[0][1] = w[0][2] = w[0][3] = 0.0;
+    w[0][4] = pp / gam1;
+#pragma unroll
+    for (int l = 1; l <= NG; ++l) {
+      w[l][0] = q[l][0];
+      w[l][1] = -q[l][1];
+      w[l][2] = -q[l][2];
+      w[l][3] = -q[l][3];
+      w[l][4] = q[l][4];
+    }
+  } else {
+    // slip wall, tangent in the x-y plane
+    const long o0 = node_off(d, i, 0, k);
+    const PrimV s = prim_of(q[1], gam1);
+    double tx = a.met[4][o0], ty = -a.met[3][o0];
+    const double J = a.met[9][o0];
+    tx *= J;
+    ty *= J;
+    const double tn = sqrt(tx * tx + ty * ty);
+    tx /= tn;
+    ty /= tn;
+#pragma unroll
+    for (int l = 1; l <= NG; ++l) {
+      const double a0 = q[l][0], a1 = q[l][1], a2 = q[l][2];
+      const double vt = a1 * tx + a2 * ty;
+      const double b1 = 2 * vt * tx - a1, b2 = 2 * vt * ty - a2;
+      w[l][0] = a0;
+      w[l][1] = b1;
+      w[l][2] = b2;
+      w[l][3] = q[l][3];
+      // the reference's energy expression, sign of the last term included
+      w[l][4] = q[l][4] - 0.5 * (a1 * a1 + a2 * a2 - b1 * b1 + b2 * b2) / a0;
+    }
+    const double vt = s.u * tx + s.v * ty;
+    const double uu = vt * tx, vv = vt * ty;
+    w[0][0] = s.r;
+    w[0][1] = s.r * uu;
+    w[0][2] = s.r * vv;
+    w[0][3] = s.r * s.w;
+    w[0][4] = s.p / gam1 + 0.5 * s.r * (uu * uu + vv * vv + s.w * s.w);
+  }
+}
+
 __global__ void bc_phase2(const BCArgs a) {
   if (a.check_done && a.st->done) return;
   const Dims& d = a.d;
@@ -158,54 +227,11 @@ __global__ void bc_phase2(const BCArgs a) {
       }
     }
   } else if (a.i_end > ui) {
-    const long o1 = node_off(d, i, 1, k), o0 = node_off(d, i, 0, k);
-    if (a.viscous) {
-      // adiabatic no-slip wall
-      const double rr = q[o1], ru = q[VOL + o1], rv = q[2 * VOL + o1], rw = q[3 * VOL + o1], rE = q[4 * VOL + o1];
-      const double pp = gam1 * (rE - 0.5 * (ru * ru + rv * rv + rw * rw) / rr);
-      put_q(a, 0, o0, rr);
-      put_q(a, 1, o0, 0.0);
-      put_q(a, 2, o0, 0.0);
-      put_q(a, 3, o0, 0.0);
-      put_q(a, 4, o0, pp / gam1);
-      for (int l = 1; l <= NG; ++l) {
-        const long s1 = node_off(d, i, l, k), g1 = node_off(d, i, -l, k);
-        put_q(a, 0, g1, q[s1]);
-        put_q(a, 1, g1, -q[VOL + s1]);
-        put_q(a, 2, g1, -q[2 * VOL + s1]);
-        put_q(a, 3, g1, -q[3 * VOL + s1]);
-        put_q(a, 4, g1, q[4 * VOL + s1]);
-      }
-    } else {
-      // slip wall, tangent in the x-y plane
-      const PrimV s = prim_of(q, o1, VOL, gam1);
-      double tx = a.met[4][o0], ty = -a.met[3][o0];
-      const double J = a.met[9][o0];
-      tx *= J;
-      ty *= J;
-      const double tn = sqrt(tx * tx + ty * ty);
-      tx /= tn;
-      ty /= tn;
-      for (int l = 1; l <= NG; ++l) {
-        const long s1 = node_off(d, i, l, k), g1 = node_off(d, i, -l, k);
-        const double a0 = q[s1], a1 = q[VOL + s1], a2 = q[2 * VOL + s1], a3 = q[3 * VOL + s1], a4 = q[4 * VOL + s1];
-        const double vt = a1 * tx + a2 * ty;
-        const double b1 = 2 * vt * tx - a1, b2 = 2 * vt * ty - a2;
-        put_q(a, 0, g1, a0);
-        put_q(a, 1, g1, b1);
-        put_q(a, 2, g1, b2);
-        put_q(a, 3, g1, a3);
-        // the reference's energy expression, sign of the last term included
-        put_q(a, 4, g1, a4 - 0.5 * (a1 * a1 + a2 * a2 - b1 * b1 + b2 * b2) / a0);
-      }
-      const double vt = s.u * tx + s.v * ty;
-      const double uu = vt * tx, vv = vt * ty;
-      put_q(a, 0, o0, s.r);
-      put_q(a, 1, o0, s.r * uu);
-      put_q(a, 2, o0, s.r * vv);
-      put_q(a, 3, o0, s.r * s.w);
-      put_q(a, 4, o0, s.p / gam1 + 0.5 * s.r * (uu * uu + vv * vv + s.w * s.w));
-    }
+    double w[NG + 1][NEQ];
+    wall_column(a, i, k, w);
+    for (int l = 0; l <= NG; ++l)
+#pragma unroll
+      for (int c = 0; c < NEQ; ++c) put_q(a, c, node_off(d, i, -l, k), w[l][c]);
   }
 }
 
@@ -442,6 +468,50 @@ __global__ void bc_farfield_batched(const BCArgs* args, const int* cta, int nblo
   farfield_body(a, ((long)blockIdx.x - __ldg(cta + lo)) * blockDim.x + threadIdx.x);
 }
 
+// The state of boundary node ob (side 0 or 1 of direction dir) from its inward
+// neighbour oe.
+__device__ __forceinline__ void characteristic_state(const BCArgs& a, int dir, int side, long ob, long oe, double qb[NEQ]) {
+  const long VOL = a.d.VOL;
+  const double mx = a.met[3 * dir][ob], my = a.met[3 * dir + 1][ob], mz = a.met[3 * dir + 2][ob];
+  const double sgn = side ? 1.0 : -1.0;
+  const double mn = sgn / sqrt(mx * mx + my * my + mz * mz);
+  const double nx = mx * mn, ny = my * mn, nz = mz * mn;
+  const PrimV se = prim_of(a.q, oe, VOL, a.gam1);
+  const double ce = sqrt(a.gamma * se.p / se.r);
+  const double qne = se.u * nx + se.v * ny + se.w * nz;
+  if (fabs(qne) >= ce && qne >= 0.0) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) qb[m] = a.q[m * VOL + oe];
+  } else {
+    double r_b, u_b, v_b, w_b, p_b;
+    const double ci = sqrt(a.gamma * a.p_inf);  // rho_inf = 1
+    const double qni = a.u_inf * nx + a.v_inf * ny;
+    if (fabs(qne) >= ce) {
+      r_b = 1.0; u_b = a.u_inf; v_b = a.v_inf; w_b = 0.0; p_b = a.p_inf;
+    } else {
+      const double rp = qne + 2.0 * ce / a.gam1, rm = qni - 2.0 * ci / a.gam1;
+      const double qnb = 0.5 * (rp + rm), cb = 0.25 * a.gam1 * (rp - rm);
+      double s, dq;
+      if (qnb >= 0.0) {
+        s = se.p / pow(se.r, a.gamma);
+        dq = qnb - qne;
+        u_b = se.u + dq * nx; v_b = se.v + dq * ny; w_b = se.w + dq * nz;
+      } else {
+        s = a.p_inf;
+        dq = qnb - qni;
+        u_b = a.u_inf + dq * nx; v_b = a.v_inf + dq * ny; w_b = dq * nz;
+      }
+      r_b = pow(cb * cb / (a.gamma * s), 1.0 / a.gam1);
+      p_b = r_b * cb * cb / a.gamma;
+    }
+    qb[0] = r_b;
+    qb[1] = r_b * u_b;
+    qb[2] = r_b * v_b;
+    qb[3] = r_b * w_b;
+    qb[4] = p_b / a.gam1 + 0.5 * r_b * (u_b * u_b + v_b * v_b + w_b * w_b);
+  }
+}
+
 // CBNS_BC_CHARACTERISTIC, one face direction per launch (dir 0 = i, 1 = j,
 // 2 = k; launched in that order).  Boundary node b, its inward neighbour e,
 // outward unit normal n = -+grad(xi_dir)/|grad(xi_dir)| at b.  Subsonic: the
@@ -473,74 +543,104 @@ __global__ void bc_characteristic(const BCArgs a, int dir, int side0, int nsides
   const long stride = dir == 0 ? 1L : dir == 1 ? d.PX : d.PL;
   const long out = side ? stride : -stride;  // offset of the next node outward
   const long ob = node_off(d, i, j, k), oe = ob - out;
-  const long VOL = d.VOL;
-  double* q = a.q;
-  const double mx = a.met[3 * dir][ob], my = a.met[3 * dir + 1][ob], mz = a.met[3 * dir + 2][ob];
-  const double sgn = side ? 1.0 : -1.0;
-  const double mn = sgn / sqrt(mx * mx + my * my + mz * mz);
-  const double nx = mx * mn, ny = my * mn, nz = mz * mn;
-  const PrimV se = prim_of(q, oe, VOL, a.gam1);
-  const double ce = sqrt(a.gamma * se.p / se.r);
-  const double qne = se.u * nx + se.v * ny + se.w * nz;
-  double qb[5];
-  if (fabs(qne) >= ce && qne >= 0.0) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) qb[m] = q[m * VOL + oe];
-  } else {
-    double r_b, u_b, v_b, w_b, p_b;
-    const double ci = sqrt(a.gamma * a.p_inf);  // rho_inf = 1
-    const double qni = a.u_inf * nx + a.v_inf * ny;
-    if (fabs(qne) >= ce) {
-      r_b = 1.0; u_b = a.u_inf; v_b = a.v_inf; w_b = 0.0; p_b = a.p_inf;
-    } else {
-      const double rp = qne + 2.0 * ce / a.gam1, rm = qni - 2.0 * ci / a.gam1;
-      const double qnb = 0.5 * (rp + rm), cb = 0.25 * a.gam1 * (rp - rm);
-      double s, dq;
-      if (qnb >= 0.0) {
-        s = se.p / pow(se.r, a.gamma);
-        dq = qnb - qne;
-        u_b = se.u + dq * nx; v_b = se.v + dq * ny; w_b = se.w + dq * nz;
-      } else {
-        s = a.p_inf;
-        dq = qnb - qni;
-        u_b = a.u_inf + dq * nx; v_b = a.v_inf + dq * ny; w_b = dq * nz;
-      }
-      r_b = pow(cb * cb / (a.gamma * s), 1.0 / a.gam1);
-      p_b = r_b * cb * cb / a.gamma;
-    }
-    qb[0] = r_b;
-    qb[1] = r_b * u_b;
-    qb[2] = r_b * v_b;
-    qb[3] = r_b * w_b;
-    qb[4] = p_b / a.gam1 + 0.5 * r_b * (u_b * u_b + v_b * v_b + w_b * w_b);
-  }
+  double qb[NEQ];
+  characteristic_state(a, dir, side, ob, oe, qb);
 #pragma unroll
   for (int l = 0; l <= NG; ++l)
 #pragma unroll
     for (int m = 0; m < 5; ++m) put_q(a, m, ob + l * out, qb[m]);
 }
 
-// CBNS_BC_OGRID, last pass: every node with i < wrap or i >= IM - wrap, the
-// i ghosts included, over the whole ghosted (j, k) box, takes Q (and in
-// viscous runs the primitives) of the node P = IM - 2*wrap away, which lies
-// on the stored periodic line and is final by now.
-__global__ void bc_wrap(const BCArgs a) {
+// CBNS_BC_OGRID in one launch: the wall on j = 0, the characteristic state on j
+// = JM-1, the k faces, and everything across the seam.  Every boundary value
+// follows from interior nodes of the P = IM - 2*wrap stored columns i = wrap ..
+// IM-wrap-1, so each is formed once, from its own column, and written to that
+// column and to its copy across the seam (the columns i < wrap and i >=
+// IM-wrap, i ghosts included, hold the column P away): no thread reads what
+// another writes.  Threads, in order: k faces (a side each), wall and far
+// columns (with the k faces of their edge nodes), then the copies of the nodes
+// no boundary condition writes (interior; ghosts off the face lines, whose
+// state is held; the primitives of j = JM+1, which phase 3 leaves as they are).
+// Four dependent launches (wall, far field, k faces, wrap) took 31 us on the
+// 384 x 128 x 4 grid, all of it launch and load latency; this one 12 (a step 337 -> 268 us).
+__global__ void __launch_bounds__(128) bc_ogrid(const BCArgs a) {
   if (a.check_done && a.st->done) return;
   const Dims& d = a.d;
-  const int W = a.wrap + NG;  // copied positions either side
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= 2L * W * d.JG * d.KG) return;
-  const int u = (int)(t % (2 * W));
-  const long r = t / (2 * W);
-  const int j = (int)(r % d.JG) - NG, k = (int)(r / d.JG) - NG;
-  const int P = d.IM - 2 * a.wrap;
-  const int i = u < W ? u - NG : d.IM - a.wrap + (u - W);
-  const int src = u < W ? i + P : i - P;
-  const long o = node_off(d, i, j, k), os = node_off(d, src, j, k);
   const long VOL = d.VOL;
+  const int W = a.wrap, P = d.IM - 2 * W, C = 2 * (W + NG);  // C: columns that have a copy
+  const int nK = P * (d.JM - 2), nJ = P * (d.KM - 2);
+  int e = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  // node (i, j, k) of a stored column and of its copies (two where P < 2 (wrap + NG))
+  auto emit = [&](int i, int j, int k, const double q[NEQ], const PrimV& s, bool prims) {
 #pragma unroll
-  for (int c = 0; c < NEQ; ++c) put_q(a, c, o, a.q[c * VOL + os]);
-  if (a.viscous) {
+    for (int m = -1; m <= 1; ++m) {
+      const int ic = i + m * P;
+      if (ic < -NG || ic > d.IM + 1) continue;
+      const long o = node_off(d, ic, j, k);
+#pragma unroll
+      for (int c = 0; c < NEQ; ++c) put_q(a, c, o, q[c]);
+      if (prims) put_prim(a, o, s);
+    }
+  };
+  const bool visc = a.viscous != 0;
+  if (e < 2 * nK) {  // k faces, j interior
+    const int side = e >= nK, r = side ? e - nK : e;
+    const int i = W + r % P, j = 1 + r / P;
+    const int src = side ? d.KM - 2 : 1, base = side ? d.KM - 1 : 0, dir = side ? 1 : -1;
+    const long os = node_off(d, i, j, src);
+    double q[NEQ];
+#pragma unroll
+    for (int c = 0; c < NEQ; ++c) q[c] = a.q[c * VOL + os];
+    PrimV s;
+    if (visc) s = prim_of(q, a.gam1);
+    for (int l = 0; l <= NG; ++l) emit(i, j, base + dir * l, q, s, visc);
+    return;
+  }
+  e -= 2 * nK;
+  if (e < 2 * nJ) {  // wall (j = 0) and far (j = JM-1) columns, k interior
+    const int far = e >= nJ, r = far ? e - nJ : e;
+    const int i = W + r % P, k = 1 + r / P;
+    double w[NG + 1][NEQ];
+    if (far) {
+      const long ob = node_off(d, i, d.JM - 1, k);
+      characteristic_state(a, 1, 1, ob, ob - d.PX, w[0]);
+#pragma unroll
+      for (int c = 0; c < NEQ; ++c) w[1][c] = w[2][c] = w[0][c];
+    } else {
+      wall_column(a, i, k, w);
+    }
+    const int j0 = far ? d.JM - 1 : 0, dj = far ? 1 : -1;
+    PrimV s;
+#pragma unroll
+    for (int l = 0; l <= NG; ++l) {
+      // primitives: all three wall nodes, JM-1 and JM of the far field
+      const bool prims = visc && !(far && l == NG);
+      if (prims) s = prim_of(w[l], a.gam1);
+      emit(i, j0 + dj * l, k, w[l], s, prims);
+      if (l == 0) {  // the k faces of the edge node
+        if (k == 1)
+          for (int m = 0; m <= NG; ++m) emit(i, j0, -m, w[0], s, visc);
+        if (k == d.KM - 2)
+          for (int m = 0; m <= NG; ++m) emit(i, j0, d.KM - 1 + m, w[0], s, visc);
+      }
+    }
+    return;
+  }
+  e -= 2 * nJ;
+  if (e >= C * d.JG * d.KG) return;
+  // copies: column u = -NG .. W-1, then IM-W .. IM+NG-1
+  const int u = e % C, r = e / C;
+  const int j = r % d.JG - NG, k = r / d.JG - NG;
+  const int i = u < W + NG ? u - NG : d.IM - W + (u - W - NG);
+  const bool kin = k >= 1 && k <= d.KM - 2, jin = j >= 1 && j <= d.JM - 2;
+  const bool held = kin ? jin : !(j >= 0 && j <= d.JM - 1);  // no boundary condition writes it
+  const bool prims = visc && (held || (kin && j == d.JM + 1));
+  const long o = node_off(d, i, j, k), os = node_off(d, u < W + NG ? i + P : i - P, j, k);
+  if (held) {
+#pragma unroll
+    for (int c = 0; c < NEQ; ++c) put_q(a, c, o, a.q[c * VOL + os]);
+  }
+  if (prims) {
 #pragma unroll
     for (int m = 0; m < 6; ++m) a.prim[m][o] = a.prim[m][os];
   }
@@ -575,17 +675,9 @@ cudaError_t launch_bc(const BCArgs& a, bool interior_prims, cudaStream_t s, int*
   }
   const long n3 = (long)d.IM * (d.KM - 2) + (long)(d.JM - 2) * (d.KM - 2) + (long)d.IM * d.JM;
   if (a.wrap) {
-    // O-grid: wall on every i of j = 0, characteristic far field on j = JM-1,
-    // the reference's k faces, then the copies across the seam
-    BCArgs w = a;
-    w.i_begin = 1u;
-    w.i_end = (unsigned)d.IM;
-    w.sigma = 0;
-    bc_phase2<<<nblk((long)d.IM * (d.KM - 2), B), B, 0, s>>>(w);
-    bc_characteristic<<<nblk((long)d.IM * (d.KM - 2), B), B, 0, s>>>(w, 1, 1, 1);
-    bc_phase3<<<nblk(n3, B), B, 0, s>>>(w);
-    bc_wrap<<<nblk(2L * (a.wrap + NG) * d.JG * d.KG, B), B, 0, s>>>(w);
-    nl += 4;
+    const long P = d.IM - 2 * a.wrap;
+    bc_ogrid<<<nblk(2 * P * (d.JM - 2) + 2 * P * (d.KM - 2) + 2L * (a.wrap + NG) * d.JG * d.KG, B), B, 0, s>>>(a);
+    ++nl;
     if (launches) *launches += nl;
     return cudaGetLastError();
   }

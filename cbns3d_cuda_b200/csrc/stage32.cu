@@ -589,6 +589,9 @@ void prepare_nb() {
 }  // namespace
 
 void stage32_prepare() {
+  static bool done = false;
+  if (done) return;
+  done = true;
   prepare_nb<2>();
   prepare_nb<3>();
 }
