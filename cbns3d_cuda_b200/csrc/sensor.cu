@@ -62,21 +62,31 @@ __global__ void sample_faces_kernel(const SampleArgs a) {
 }
 
 // ---------------------------------------------------------------- loss and gradient
-constexpr int TILE = 128, GT = 256, HP = SN_H + 1;
+constexpr int TILE = 64, GT = 256;
+constexpr int HP = SN_H + 4, XP = 20;  // row pitches: 16-byte rows, four rows apart in different banks
+
+static_assert(TILE * HP > SP_N && TILE * XP >= SN_H * 16, "the gradients fit the tile's buffers");
 
 struct GradSmem {
-  float x[TILE][16];
-  float h1[TILE][HP], h2[TILE][HP], g2[TILE][HP], g1[TILE][HP];
+  alignas(16) float x[TILE][XP];
+  alignas(16) float h1[TILE][HP], h2[TILE][HP], g2[TILE][HP], g1[TILE][HP];
+  alignas(16) float W2[SN_H][HP];
   float dz[TILE];
-  float W2[SN_H][SN_H];
   float w3[SN_H];
 };
 
 // Binary cross-entropy with positive-class weight, averaged over n samples:
 // loss = -(1/n) sum w_i [y_i log p_i + (1 - y_i) log(1 - p_i)], p = sigmoid(z).
-// Each CTA takes tiles of 128 samples: forward into shared memory, backward by
+// Each CTA takes tiles of 64 samples: forward into shared memory, backward by
 // the chain rule, per-thread partial sums of the weight gradients in registers,
-// one atomic add per parameter per CTA at the end.
+// one atomic add per parameter per CTA at the end.  Bound by the latency of a
+// tile's chain of phases: a training batch (16,384 samples) is one tile for each
+// of 256 CTAs, so the tile is small, rows are read as float4 (broadcast), the
+// weight gradients take 2 x 2 outputs per thread (two 8-byte reads for four
+// products) and the last layer shares its sums among four threads a row.
+// 16,384 samples: 20.3 -> 14.2 us (128 tiles of 128 samples before; weights
+// loaded across their rows), 1.5 M samples 1050 -> 696 us; summing over clusters
+// of 4 or 8 CTAs first was slower (15.0 and 17.7 us, 1213 us).
 __global__ void __launch_bounds__(GT) mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
                                                       const unsigned char* __restrict__ Y, unsigned n, float pos_w,
                                                       float inv_n, float* G, float* loss) {
@@ -84,123 +94,201 @@ __global__ void __launch_bounds__(GT) mlp_grad_kernel(const float* __restrict__ 
   GradSmem& s = *reinterpret_cast<GradSmem*>(raw);
   const int t = threadIdx.x;
   const int c = t & 31, rb = t >> 5;  // column and first row of this thread's outputs
+  // the weights through shared memory (a thread's rows of them straight from
+  // memory are 47 loads of 32 sectors each, 6 us a CTA)
   for (int e = t; e < SN_H * SN_H; e += GT) s.W2[e / SN_H][e % SN_H] = P[SP_W2 + e];
-  if (t < SN_H) s.w3[t] = P[SP_W3 + t];
-  float w1[SN_IN], w2[SN_H];
-#pragma unroll
-  for (int k = 0; k < SN_IN; ++k) w1[k] = P[SP_W1 + c * SN_IN + k];
-#pragma unroll
-  for (int k = 0; k < SN_H; ++k) w2[k] = P[SP_W2 + c * SN_H + k];
-  const float b1 = P[SP_B1 + c], b2 = P[SP_B2 + c], b3 = P[SP_B3];
-  // owned gradient entries
-  float gW2[4] = {0, 0, 0, 0}, gW1[2] = {0, 0}, gvec = 0.f, lsum = 0.f;
+  for (int e = t; e < SN_H * SN_IN; e += GT) s.x[e / SN_IN][e % SN_IN] = P[SP_W1 + e];
+  if (t < SN_H) {
+    s.w3[t] = P[SP_W3 + t];
+    s.x[t][SN_IN] = 0.f;
+  }
   __syncthreads();
+  float w1[SN_IN + 1], w2[SN_H];
+#pragma unroll
+  for (int k = 0; k < SN_IN + 1; ++k) w1[k] = s.x[c][k];
+#pragma unroll
+  for (int k = 0; k < SN_H; ++k) w2[k] = s.W2[c][k];
+  const float b1 = P[SP_B1 + c], b2 = P[SP_B2 + c], b3 = P[SP_B3];
+  // owned gradient entries: a 2 x 2 block of W2 (rows 2i.., columns 2j..), of W1
+  // (columns below 15; threads below 128), and one entry of the vectors
+  const int bi = 2 * (t >> 4), bj = 2 * (t & 15);
+  const int ai = 2 * ((t & 127) >> 3), aj = 2 * (t & 7);
+  float gW2[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, gW1[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, gvec = 0.f, lsum = 0.f;
+  __syncthreads();
+  auto dot4 = [](const float4 a, const float* w, float h) {
+    h += a.x * w[0];
+    h += a.y * w[1];
+    h += a.z * w[2];
+    return h + a.w * w[3];
+  };
   const unsigned ntiles = (n + TILE - 1) / TILE;
   for (unsigned tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned base = tile * TILE;
-    for (int e = t; e < TILE * 16; e += GT) {
-      const int r = e >> 4, k = e & 15;
-      const unsigned sidx = base + r;
-      s.x[r][k] = (k < SN_IN && sidx < n) ? X[(size_t)sidx * SN_IN + k] : 0.f;
+    for (int e = t; e < TILE * SN_IN; e += GT) {  // the tile's features are contiguous
+      const int r = e / SN_IN, k = e % SN_IN;
+      s.x[r][k] = base + r < n ? X[(size_t)base * SN_IN + e] : 0.f;
     }
+    if (t < TILE) s.x[t][SN_IN] = 0.f;
     __syncthreads();
-    for (int r = rb; r < TILE; r += 8) {
+#pragma unroll 4
+    for (int r = rb; r < TILE; r += GT / 32) {
+      const float4* xr = reinterpret_cast<const float4*>(s.x[r]);
       float h = b1;
 #pragma unroll
-      for (int k = 0; k < SN_IN; ++k) h += s.x[r][k] * w1[k];
+      for (int k = 0; k < 4; ++k) h = dot4(xr[k], w1 + 4 * k, h);
       s.h1[r][c] = fmaxf(h, 0.f);
     }
     __syncthreads();
-    for (int r = rb; r < TILE; r += 8) {
+#pragma unroll 4
+    for (int r = rb; r < TILE; r += GT / 32) {
+      const float4* hr = reinterpret_cast<const float4*>(s.h1[r]);
       float h = b2;
 #pragma unroll
-      for (int k = 0; k < SN_H; ++k) h += s.h1[r][k] * w2[k];
+      for (int k = 0; k < SN_H / 4; ++k) h = dot4(hr[k], w2 + 4 * k, h);
       s.h2[r][c] = fmaxf(h, 0.f);
     }
     __syncthreads();
-    if (t < TILE) {
-      const unsigned sidx = base + t;
-      float dz = 0.f;
-      if (sidx < n) {
-        float z = b3;
+    {  // the logit, loss and its derivative: row t / 4, a quarter of the sum each
+      const int r = t >> 2, q = t & 3;
+      const unsigned sidx = base + r;
+      float z = 0.f;
 #pragma unroll
-        for (int k = 0; k < SN_H; ++k) z += s.h2[t][k] * s.w3[k];
-        const float y = Y[sidx] ? 1.f : 0.f;
-        const float w = Y[sidx] ? pos_w : 1.f;
-        const float p = 1.f / (1.f + __expf(-z));
-        // log(sigmoid(z)) and log(1 - sigmoid(z)) in a form that does not overflow
-        const float lp = -log1pf(__expf(-fabsf(z))) + fminf(z, 0.f);
-        const float lq = lp - z;
-        lsum += -w * (y * lp + (1.f - y) * lq) * inv_n;
-        dz = w * (p - y) * inv_n;
+      for (int k = 0; k < SN_H / 4; ++k) z += s.h2[r][4 * k + q] * s.w3[4 * k + q];
+      z += __shfl_xor_sync(0xffffffffu, z, 1);
+      z += __shfl_xor_sync(0xffffffffu, z, 2);
+      z += b3;
+      if (q == 0) {
+        float dz = 0.f;
+        if (sidx < n) {
+          const float y = Y[sidx] ? 1.f : 0.f;
+          const float w = Y[sidx] ? pos_w : 1.f;
+          const float p = 1.f / (1.f + __expf(-z));
+          // log(sigmoid(z)) and log(1 - sigmoid(z)) in a form that does not overflow
+          const float lp = -log1pf(__expf(-fabsf(z))) + fminf(z, 0.f);
+          const float lq = lp - z;
+          lsum += -w * (y * lp + (1.f - y) * lq) * inv_n;
+          dz = w * (p - y) * inv_n;
+        }
+        s.dz[r] = dz;
       }
-      s.dz[t] = dz;
     }
     __syncthreads();
-    for (int r = rb; r < TILE; r += 8) s.g2[r][c] = s.h2[r][c] > 0.f ? s.dz[r] * s.w3[c] : 0.f;
+    for (int r = rb; r < TILE; r += GT / 32) s.g2[r][c] = s.h2[r][c] > 0.f ? s.dz[r] * s.w3[c] : 0.f;
     __syncthreads();
     // dW2[cc][k] = sum_r g2[r][cc] h1[r][k]
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = t + GT * q, cc = e / SN_H, k = e % SN_H;
-      float acc = 0.f;
-      for (int r = 0; r < TILE; ++r) acc += s.g2[r][cc] * s.h1[r][k];
-      gW2[q] += acc;
+    {
+      float a00 = 0.f, a01 = 0.f, a10 = 0.f, a11 = 0.f;
+#pragma unroll 8
+      for (int r = 0; r < TILE; ++r) {
+        const float2 g = *reinterpret_cast<const float2*>(&s.g2[r][bi]), h = *reinterpret_cast<const float2*>(&s.h1[r][bj]);
+        a00 += g.x * h.x;
+        a01 += g.x * h.y;
+        a10 += g.y * h.x;
+        a11 += g.y * h.y;
+      }
+      gW2[0][0] += a00;
+      gW2[0][1] += a01;
+      gW2[1][0] += a10;
+      gW2[1][1] += a11;
     }
-    // per-column vectors: db1 (t<32, after g1), db2 (32..63), dw3 (64..95), db3 (96)
+    // per-column vectors: db2 (32..63), dw3 (64..95), db3 (96); db1 after g1
     if (t >= 32 && t < 64) {
       float acc = 0.f;
+#pragma unroll 8
       for (int r = 0; r < TILE; ++r) acc += s.g2[r][t - 32];
       gvec += acc;
     } else if (t >= 64 && t < 96) {
       float acc = 0.f;
+#pragma unroll 8
       for (int r = 0; r < TILE; ++r) acc += s.dz[r] * s.h2[r][t - 64];
       gvec += acc;
     } else if (t == 96) {
       float acc = 0.f;
+#pragma unroll 8
       for (int r = 0; r < TILE; ++r) acc += s.dz[r];
       gvec += acc;
     }
     // g1[r][k] = (sum_c g2[r][c] W2[c][k]) * relu'(h1)
-    for (int r = rb; r < TILE; r += 8) {
-      float acc = 0.f;
+    {
+      float w2c[SN_H];
 #pragma unroll
-      for (int cc = 0; cc < SN_H; ++cc) acc += s.g2[r][cc] * s.W2[cc][c];
-      s.g1[r][c] = s.h1[r][c] > 0.f ? acc : 0.f;
+      for (int cc = 0; cc < SN_H; ++cc) w2c[cc] = s.W2[cc][c];
+#pragma unroll 4
+      for (int r = rb; r < TILE; r += GT / 32) {
+        const float4* gr = reinterpret_cast<const float4*>(s.g2[r]);
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < SN_H / 4; ++k) acc = dot4(gr[k], w2c + 4 * k, acc);
+        s.g1[r][c] = s.h1[r][c] > 0.f ? acc : 0.f;
+      }
     }
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int e = t + GT * q;
-      if (e < SN_H * SN_IN) {
-        const int cc = e / SN_IN, k = e % SN_IN;
-        float acc = 0.f;
-        for (int r = 0; r < TILE; ++r) acc += s.g1[r][cc] * s.x[r][k];
-        gW1[q] += acc;
+    // dW1, by two halves of the rows (threads 0..127 and 128..255)
+    {
+      const int r0 = t < 128 ? 0 : TILE / 2;
+      float a00 = 0.f, a01 = 0.f, a10 = 0.f, a11 = 0.f;
+#pragma unroll 8
+      for (int r = r0; r < r0 + TILE / 2; ++r) {
+        const float2 g = *reinterpret_cast<const float2*>(&s.g1[r][ai]), x = *reinterpret_cast<const float2*>(&s.x[r][aj]);
+        a00 += g.x * x.x;
+        a01 += g.x * x.y;
+        a10 += g.y * x.x;
+        a11 += g.y * x.y;
       }
+      gW1[0][0] += a00;
+      gW1[0][1] += a01;
+      gW1[1][0] += a10;
+      gW1[1][1] += a11;
     }
     if (t < 32) {
       float acc = 0.f;
+#pragma unroll 8
       for (int r = 0; r < TILE; ++r) acc += s.g1[r][t];
       gvec += acc;
     }
     __syncthreads();
   }
+  // the CTA's gradients (and the loss at index SP_N) through shared memory, so
+  // that neighbouring threads add to neighbouring parameters
+  float* own = &s.h1[0][0];  // TILE x HP >= SP_N + 1 floats; the loop's last barrier freed it
 #pragma unroll
-  for (int q = 0; q < 4; ++q) atomicAdd(&G[SP_W2 + t + GT * q], gW2[q]);
+  for (int p = 0; p < 2; ++p)
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-    if (t + GT * q < SN_H * SN_IN) atomicAdd(&G[SP_W1 + t + GT * q], gW1[q]);
-  if (t < 32) atomicAdd(&G[SP_B1 + t], gvec);
-  else if (t < 64) atomicAdd(&G[SP_B2 + t - 32], gvec);
-  else if (t < 96) atomicAdd(&G[SP_W3 + t - 64], gvec);
-  else if (t == 96) atomicAdd(&G[SP_B3], gvec);
-  if (t < TILE) {
-    float l = lsum;
+    for (int q = 0; q < 2; ++q) own[SP_W2 + (bi + p) * SN_H + bj + q] = gW2[p][q];
+  if (t >= 128) {  // the second half of the rows' share of W1
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((t & 31) == 0) atomicAdd(loss, l);
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) s.x[0][(ai + p) * 16 + aj + q] = gW1[p][q];
   }
+  if (t < 32) own[SP_B1 + t] = gvec;
+  else if (t < 64) own[SP_B2 + t - 32] = gvec;
+  else if (t < 96) own[SP_W3 + t - 64] = gvec;
+  else if (t == 96) own[SP_B3] = gvec;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  if ((t & 31) == 0) s.dz[t >> 5] = lsum;
+  __syncthreads();
+  if (t < 128) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (aj + q < SN_IN) own[SP_W1 + (ai + p) * SN_IN + aj + q] = gW1[p][q] + s.x[0][(ai + p) * 16 + aj + q];
+  }
+  if (t == 0) {
+    float l = 0.f;
+    for (int w = 0; w < GT / 32; ++w) l += s.dz[w];
+    own[SP_N] = l;
+  }
+  __syncthreads();
+  for (int e = t; e <= SP_N; e += GT) atomicAdd(e < SP_N ? G + e : loss, own[e]);
+}
+
+__global__ void zero_grad(float* G, float* loss) {
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  if (e < SP_N) G[e] = 0.f;
+  else if (e == SP_N) *loss = 0.f;
 }
 
 // ---------------------------------------------------------------- widening
@@ -444,8 +532,8 @@ cudaError_t launch_sensor_dilate_batched(const DilateArgs* args, const int* cta,
 
 cudaError_t launch_mlp_grad(const float* P, const float* X, const unsigned char* Y, unsigned n, float pos_w, float* G,
                             float* loss, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(G, 0, SP_N * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(loss, 0, sizeof(float), s);
+  zero_grad<<<(SP_N + 256) / 256, 256, 0, s>>>(G, loss);  // one launch for two memsets
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
   static bool attr = false;
