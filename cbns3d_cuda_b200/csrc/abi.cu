@@ -292,16 +292,19 @@ ViscArgs visc_args(cbns_ctx* c, bool check_done, bool sigma) {
   a.dt_full = c->prm.dt_viscous == CBNS_DTV_FULL;
   a.qc = -c->ph.Pr_inv * c->ph.gam1_inv / c->ph.Mach2;
   for (int m = 0; m < 6; ++m) a.prim[m] = c->f.prim[m];
-  fill_met(c, a.met);
+  for (int m = 0; m < 10; ++m) a.area[m] = c->f.area[m];
+  for (int m = 0; m < 9; ++m) a.area32[m] = c->f.area32[m];
+  a.Mach_inv = 1.0 / c->prm.Mach;
   for (int m = 0; m < 12; ++m) a.vflux[m] = c->f.vflux[m];
   for (int m = 0; m < 4; ++m) a.dfv[m] = c->f.dfv[m];
   a.f32 = c->ph.precision != CBNS_PREC_FP64;
   a.visdiv = c->ph.visdiv;
   a.mu = c->f.prim[6];
+  a.keep_mu = sigma || !check_done;
   a.st = c->st;
   a.check_done = check_done;
   a.sigma = sigma;
-  a.kc = visc_kchunk(c->d, c->nsm);
+  a.kc = visc_kchunk(c->d, c->nsm, a.f32, false);
   return a;
 }
 
@@ -328,6 +331,7 @@ StageArgs stage_args(cbns_ctx* c, const double* src, const double* q0, const dou
   a.kchunk = c->kchunk;
   a.visdiv = c->ph.visdiv;
   a.sigma = sigma;
+  a.lean = 0;
   a.mask = c->ph.precision == CBNS_PREC_HYBRID ? c->mask : nullptr;
   a.wflux = c->wflux;
   a.tm = c->tm[0];  // src, q0 and qp are state buffers (or q0, qp null: RHS only)
@@ -545,7 +549,9 @@ int enqueue_step(cbns_ctx* c) {
     // O-grid: the wrap copy rewrites nodes stage 3 updated, so the spectral
     // radius is swept after the boundary pass
     const bool fuse = last && !visc && !ogrid(c);
-    RET(stage_launch(c, stage_args(c, s[k].src, s[k].q0, s[k].qp, s[k].out, fuse), k + 1));
+    StageArgs sa = stage_args(c, s[k].src, s[k].q0, s[k].qp, s[k].out, fuse);
+    sa.lean = !last;
+    RET(stage_launch(c, sa, k + 1));
     // no boundary pass in the step for a viscous far-field block: its
     // boundary and ghost nodes hold their Q, so their primitives (formed at
     // the start of the run) stand, the stage kernel recovering the interior
@@ -775,7 +781,10 @@ int batch_tables(cbns_batch* b) {
     // the batch's own chunking instead of each block's (sized for the block
     // alone on the whole GPU)
     const int kc = std::min(c->d.KM - 2, kBatchKChunk);
-    for (int r = 0; r < 3; ++r) tab[r * nb + i].kchunk = kc;
+    for (int r = 0; r < 3; ++r) {
+      tab[r * nb + i].kchunk = kc;
+      tab[r * nb + i].lean = r < 2;
+    }
     start[i + 1] = start[i] + c->ntile_i * c->ntile_j * ((c->d.KM - 2 + kc - 1) / kc);
     b->roles.insert(b->roles.end(), {c->lq, c->lp, c->ls});
   }
@@ -796,7 +805,10 @@ int batch_tables(cbns_batch* b) {
     for (int k = 0; k < 3; ++k) {
       double* out = k == 0 ? c->qb[c->ls] : (k == 1 ? c->qb[c->lp] : c->qb[c->lq]);
       bct[k * nb + i] = bc_args(c, out, true, k == 2 && !b->visc);
-      if (b->visc) vt[k * nb + i] = visc_args(c, true, k == 2);
+      if (b->visc) {
+        vt[k * nb + i] = visc_args(c, true, k == 2);
+        vt[k * nb + i].kc = visc_kchunk(c->d, c->nsm, b->fp32, true);
+      }
     }
     bcc[i + 1] = bcc[i] + bc_farfield_ctas(c->d);
     vc[i + 1] = vc[i] + (b->visc ? visc_ctas(vt[i]) : 0);

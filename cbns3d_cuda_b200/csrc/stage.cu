@@ -460,12 +460,12 @@ __device__ __forceinline__ void stage_body(const StageCore& a, const StageMaps* 
           const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
           const double ke = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
           const double pp = __dmul_rn(a.gam1, __fma_rn(-__dmul_rn(0.5, r), ke, q[4]));
-          a.prim[0][o] = r;
+          if (!a.lean) a.prim[0][o] = r;
           a.prim[1][o] = uu;
           a.prim[2][o] = vv;
           a.prim[3][o] = ww;
-          a.prim[4][o] = pp;
-          a.prim[5][o] = a.gM2 * pp / r;
+          if (!a.lean) a.prim[4][o] = pp;
+          a.prim[5][o] = ml(ml(a.gM2, pp), ir);
         } else if (kSigma && a.sigma) {
           // in FP64 only where the FP32 bound reaches the largest met so far
           float qf[NEQ], small;

@@ -39,6 +39,7 @@ struct StageCore {
   int q0_is_src, qp_is_src;  // RK operands that equal the stage input (read from the ring)
   int ntile_i, ntile_j, kchunk;
   int visdiv;          // CBNS_VISDIV_*
+  int lean;            // viscous, stages 1 and 2 of a run: rho and p of the primitives are not read before stage 3
   int sigma;           // accumulate the interior spectral-radius max (inviscid stage 3)
 };
 struct StageArgs : StageCore {

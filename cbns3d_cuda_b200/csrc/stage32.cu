@@ -417,12 +417,12 @@ __device__ __forceinline__ void stage32_body(const StageCore& a, const StageMaps
           const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
           const double kk = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
           const double pp = __dmul_rn(a.gam1, __fma_rn(-__dmul_rn(0.5, r), kk, q[4]));
-          a.prim[0][o] = r;
+          if (!a.lean) a.prim[0][o] = r;
           a.prim[1][o] = uu;
           a.prim[2][o] = vv;
           a.prim[3][o] = ww;
-          a.prim[4][o] = pp;
-          a.prim[5][o] = a.gM2 * pp / r;
+          if (!a.lean) a.prim[4][o] = pp;
+          a.prim[5][o] = ml(ml(a.gM2, pp), ir);
         }
       }
     }

@@ -21,6 +21,10 @@
 // stage kernel's latency-bound update.
 #include "visc.cuh"
 
+#include <algorithm>
+
+#include "sigma.cuh"
+
 namespace cbns {
 
 namespace {
@@ -42,8 +46,9 @@ static_assert(VHALO <= VT, "one halo node per thread");
 // float for the FP32-flux precisions)
 template <typename T>
 struct ViscSmem {
-  T c[4][CJ][CW];            // plane k with its halo (corners unused)
+  T c[2][4][CJ][CW];         // plane p with its halo (corners unused) in buffer p & 1
   T ring[VR][4][VTJ][VTI];   // the tile on planes k-2 .. k+2, slot = plane mod 5
+  int best;                  // the largest spectral radius met so far (sigma.cuh)
 };
 
 // derivative from the values v(-3) .. v(+3) along the axis (only those the
@@ -121,18 +126,22 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
   auto put_plane = [&](int p, const T h[4]) {  // c <- plane p: halo from h, the tile from the ring
     if (hin) {
 #pragma unroll
-      for (int f = 0; f < 4; ++f) sm.c[f][hcy][hcx] = h[f];
+      for (int f = 0; f < 4; ++f) sm.c[p & 1][f][hcy][hcx] = h[f];
     }
     if (own) {
 #pragma unroll
-      for (int f = 0; f < 4; ++f) sm.c[f][VH + ty][VH + tx] = sm.ring[p % VR][f][ty][tx];
+      for (int f = 0; f < 4; ++f) sm.c[p & 1][f][VH + ty][VH + tx] = sm.ring[p % VR][f][ty][tx];
     }
   };
 
-  // warm-up: the ring on planes kb-2 .. kb+2, plane kb in c
-  for (int p = kb - 2; p <= kb + 2; ++p) {
-    load_ring(p, rn);
-    put_ring(p, rn);
+  // warm-up: the ring on planes kb-2 .. kb+2, all loads in flight, plane kb in c
+  if (a.sigma && t == 0) sm.best = __float_as_int(sigma_start(a.st));
+  {
+    T w[VR][4];
+#pragma unroll
+    for (int p = 0; p < VR; ++p) load_ring(kb - 2 + p, w[p]);
+#pragma unroll
+    for (int p = 0; p < VR; ++p) put_ring(kb - 2 + p, w[p]);
   }
   load_halo(kb, hn);
   put_plane(kb, hn);
@@ -148,15 +157,21 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
     }
     if (valid) {
       const long o = o_own + k * sk;
+      // the node's area vectors J*grad(xi|eta|zeta) and 1/J: the gradients'
+      // chain rule takes 1/J into the viscosity, the fluxes' normals are the
+      // area vectors themselves
       T m9[9];
 #pragma unroll
-      for (int m = 0; m < 9; ++m) m9[m] = (T)__ldg(a.met[m] + o);
-      const T J = (T)__ldg(a.met[9] + o);
+      for (int m = 0; m < 9; ++m) {
+        if constexpr (sizeof(T) == 4) m9[m] = __ldg(a.area32[m] + o);
+        else m9[m] = __ldg(a.area[m] + o);
+      }
+      const T iJ = (T)__ldg(a.area[9] + o);
       T gx[4], ge[4], gz[4];
       const int s0 = (k + VR - 2) % VR, s1 = (k + VR - 1) % VR, s3 = (k + 1) % VR, s4 = (k + 2) % VR;
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        const T (*cp)[CW] = sm.c[f];
+        const T (*cp)[CW] = sm.c[k & 1][f];
         const int y = VH + ty, x = VH + tx;
         gx[f] = dgv<T>([&](int q) { return cp[y][x + q]; }, gi, IG);
         ge[f] = dgv<T>([&](int q) { return cp[y + q][x]; }, gj, JG);
@@ -175,11 +190,12 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
             },
             k, KG);
       }
-      const T uu = sm.c[0][VH + ty][VH + tx], vv = sm.c[1][VH + ty][VH + tx], ww = sm.c[2][VH + ty][VH + tx];
-      const T Tl = sm.c[3][VH + ty][VH + tx];
+      const T (*c4)[CJ][CW] = sm.c[k & 1];
+      const T uu = c4[0][VH + ty][VH + tx], vv = c4[1][VH + ty][VH + tx], ww = c4[2][VH + ty][VH + tx];
+      const T Tl = c4[3][VH + ty][VH + tx];
       const T CT = (T)a.C_T_inf;
-      const T mu = (T(1) + CT) / (Tl + CT) * sqrt(Tl * Tl * Tl);
-      a.mu[o] = (double)mu;
+      const T mu = ml((T(1) + CT) * Tl * sqrt_(Tl), rcp_(Tl + CT));
+      if (a.keep_mu) a.mu[o] = (double)mu;
       // chain rule: d/dx = xi_x d/dxi + eta_x d/deta + zeta_x d/dzeta, etc.
       const T ux = gx[0] * m9[0] + ge[0] * m9[3] + gz[0] * m9[6];
       const T uy = gx[0] * m9[1] + ge[0] * m9[4] + gz[0] * m9[7];
@@ -190,7 +206,7 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
       const T wx = gx[2] * m9[0] + ge[2] * m9[3] + gz[2] * m9[6];
       const T wy = gx[2] * m9[1] + ge[2] * m9[4] + gz[2] * m9[7];
       const T wz = gx[2] * m9[2] + ge[2] * m9[5] + gz[2] * m9[8];
-      const T mr = mu * (T)a.Re_inv;
+      const T mr = mu * (T)a.Re_inv * iJ;
       const T txx = T(2.0 / 3.0) * mr * (T(2) * ux - vy - wz);
       const T tyy = T(2.0 / 3.0) * mr * (T(2) * vy - ux - wz);
       const T tzz = T(2.0 / 3.0) * mr * (T(2) * wz - ux - vy);
@@ -204,7 +220,7 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
       const T ez = uu * txz + vv * tyz + ww * tzz - qz;
 #pragma unroll
       for (int dd = 0; dd < 3; ++dd) {
-        const T nx = m9[3 * dd] * J, ny = m9[3 * dd + 1] * J, nz = m9[3 * dd + 2] * J;
+        const T nx = m9[3 * dd], ny = m9[3 * dd + 1], nz = m9[3 * dd + 2];
         reinterpret_cast<V*>(a.vflux[4 * dd + 0])[o] = nx * txx + ny * txy + nz * txz;
         reinterpret_cast<V*>(a.vflux[4 * dd + 1])[o] = nx * txy + ny * tyy + nz * tyz;
         reinterpret_cast<V*>(a.vflux[4 * dd + 2])[o] = nx * txz + ny * tyz + nz * tzz;
@@ -212,31 +228,49 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
       }
       const int i = gi - NG, j = gj - NG, kk = k - NG;
       if (a.sigma && i >= 0 && i < d.IM && j >= 0 && j < d.JM && kk >= 0 && kk < d.KM) {
-        // the spectral radius for the next dt, in FP64 from the FP64 fields
-        // whatever T is (src/time_step_kernel.cu:13-96)
-        const double rr = __ldg(a.prim[0] + o), pp = __ldg(a.prim[4] + o);
-        const bool t64 = sizeof(T) == 8;
-        const double ud = t64 ? (double)uu : __ldg(a.prim[1] + o), vd = t64 ? (double)vv : __ldg(a.prim[2] + o),
-                     wd = t64 ? (double)ww : __ldg(a.prim[3] + o), Td = t64 ? (double)Tl : __ldg(a.prim[5] + o);
-        const double mud = t64 ? (double)mu : (1.0 + a.C_T_inf) / (Td + a.C_T_inf) * sqrt(Td * Td * Td);
-        const double c = sqrt(a.gamma * pp / rr);
-        const double fv = a.dt_full ? 2.0 * mud * a.C_dt_v / rr
-                                    : 2.0 * mud * a.C_dt_v * sqrt(ud * ud + vd * vd + wd * wd) / c / rr;
-        double s = 0.0;
+        // the spectral radius for the next dt (src/time_step_kernel.cu:13-96):
+        // FP64 from the FP64 fields, where an FP32 bound of it (rounded values,
+        // c = sqrt(T)/M; the roundings covered by 1e-6 |u||A| and 2e-5) reaches
+        // the largest met so far
+        const float fu = (float)uu, fv = (float)vv, fw = (float)ww, ft = (float)Tl, fi = fabsf((float)iJ);
+        const float ir = rcp_((float)__ldg(a.prim[0] + o));
+        const float qm = fabsf(fu) + fabsf(fv) + fabsf(fw);
+        const float c = sqrt_(ft) * (float)a.Mach_inv;
+        const float vis = 2.f * (float)mu * (float)a.C_dt_v * ir * (a.dt_full ? 1.f : qm * rcp_(c)) * fi;
+        float b = 0.f, small = 1.f;
 #pragma unroll
         for (int dd = 0; dd < 3; ++dd) {
-          const double mx = t64 ? (double)m9[3 * dd] : __ldg(a.met[3 * dd] + o);
-          const double my = t64 ? (double)m9[3 * dd + 1] : __ldg(a.met[3 * dd + 1] + o);
-          const double mz = t64 ? (double)m9[3 * dd + 2] : __ldg(a.met[3 * dd + 2] + o);
-          const double na = sqrt(mx * mx + my * my + mz * mz);
-          s += fabs(ud * mx + vd * my + wd * mz) + c * na + na * na * fv;
+          const float x = (float)m9[3 * dd], y = (float)m9[3 * dd + 1], z = (float)m9[3 * dd + 2];
+          const float nn = fm(z, z, fm(y, y, ml(x, x)));
+          small = fminf(small, nn);
+          b += fabsf(fm(fw, z, fm(fv, y, ml(fu, x)))) + fm(1.0e-6f, qm, c) * sqrt_(nn) + nn * vis;
         }
-        if (s != s) nanseen = true;
-        else if (!has || s > sg) sg = s;
-        has = true;
+        b *= fi * (1.f + 2.0e-5f);
+        if (sigma_reaches(b, small, __int_as_float(*(volatile int*)&sm.best))) {
+          const double ud = __ldg(a.prim[1] + o), vd = __ldg(a.prim[2] + o), wd = __ldg(a.prim[3] + o);
+          const double Td = __ldg(a.prim[5] + o), ird = rcp_(__ldg(a.prim[0] + o));
+          const double J1 = fabs(__ldg(a.area[9] + o));
+          const double cd = sqrt_(a.gamma * __ldg(a.prim[4] + o) * ird);
+          const double mud = (1.0 + a.C_T_inf) * Td * sqrt_(Td) * rcp_(Td + a.C_T_inf);
+          const double fvd = 2.0 * mud * a.C_dt_v * ird * (a.dt_full ? 1.0 : sqrt_(ud * ud + vd * vd + wd * wd) * rcp_(cd));
+          double s = 0.0;
+#pragma unroll 1
+          for (int dd = 0; dd < 3; ++dd) {
+            const double mx = __ldg(a.area[3 * dd] + o), my = __ldg(a.area[3 * dd + 1] + o),
+                         mz = __ldg(a.area[3 * dd + 2] + o);
+            const double nn = mx * mx + my * my + mz * mz;
+            s += fabs(ud * mx + vd * my + wd * mz) + cd * sqrt_(nn) + nn * J1 * fvd;
+          }
+          s *= J1;
+          if (s != s) nanseen = true;
+          else if (!has || s > sg) sg = s;
+          has = true;
+          sigma_found(&sm.best, s);
+        }
       }
     }
-    __syncthreads();  // plane k and ring slot k-2 are no longer read
+    // the ring is the thread's own column, plane k+1's buffer was last read
+    // for plane k-1: one barrier per plane
     if (more) {
       put_ring(k + 3, rn);
       put_plane(k + 1, hn);
@@ -300,7 +334,7 @@ __global__ void __launch_bounds__(256) visc_div_batched(const ViscArgs* args, co
 }
 
 template <typename V>
-__global__ void __launch_bounds__(VT, sizeof(V) == 4 ? 3 : 2) visc_node_kernel(const ViscArgs a) {
+__global__ void __launch_bounds__(VT, sizeof(V) == 4 ? 4 : 2) visc_node_kernel(const ViscArgs a) {
   if (a.check_done && a.st->done) return;
   extern __shared__ __align__(16) unsigned char vraw[];
   visc_node_tile<V>(a, blockIdx.x, *reinterpret_cast<ViscSmem<V>*>(vraw));
@@ -309,7 +343,7 @@ __global__ void __launch_bounds__(VT, sizeof(V) == 4 ? 3 : 2) visc_node_kernel(c
 // Many blocks in one launch: block b owns CTAs cta[b] .. cta[b+1]-1, args[b]
 // are its ViscArgs.
 template <typename V>
-__global__ void __launch_bounds__(VT, sizeof(V) == 4 ? 3 : 2) visc_node_batched(const ViscArgs* args, const int* cta,
+__global__ void __launch_bounds__(VT, sizeof(V) == 4 ? 4 : 2) visc_node_batched(const ViscArgs* args, const int* cta,
                                                                                int nblocks) {
   const int lo = block_of_cta(cta, nblocks, (int)blockIdx.x);
   const ViscArgs& a = args[lo];
@@ -353,15 +387,30 @@ int visc_div_ctas(const Dims& d) {
   return (int)((n + 255) / 256);
 }
 
-int visc_kchunk(const Dims& d, int nsm) {
-  // chunks enough for about four waves of 2 CTAs per SM, at least 16 planes
-  // each (each chunk loads 5 planes ahead of its first)
+// A chunk takes its planes plus about 2.5 for its start (five ring planes
+// loaded ahead of its first).  At least 16 planes where that makes at least
+// two waves of CTAs (batch: always, the blocks sharing the launch); otherwise
+// the chunk whose waves (half a chunk of tail where there is more than one) are
+// shortest: on 128x64x64 FP64 11 planes (270 CTAs, one wave) instead of 16 (225)
+// take 47.7 us per launch instead of 64.6.
+int visc_kchunk(const Dims& d, int nsm, bool f32, bool batch) {
   const int VK = d.KG - 2;
   const long tiles = (long)((d.IG - 2 + VTI - 1) / VTI) * ((d.JG - 2 + VTJ - 1) / VTJ);
   const long want = (8L * nsm + tiles - 1) / tiles;
-  int kc = (int)((VK + want - 1) / want);
-  if (kc < 16) kc = 16;
-  return kc < VK ? kc : VK;
+  const int long_kc = std::min(VK, std::max(16, (int)((VK + want - 1) / want)));
+  const double slots = (double)nsm * (f32 ? 4 : 2);
+  if (batch || tiles * ((VK + long_kc - 1) / long_kc) >= 2 * slots) return long_kc;
+  double best = 1e300;
+  int best_k = long_kc;
+  for (int kc = 1; kc <= VK; ++kc) {
+    const double items = (double)tiles * ((VK + kc - 1) / kc), chunk = kc + 2.5;
+    const double cost = items <= slots ? chunk : (items / slots + 0.5) * chunk;
+    if (cost < best - 1e-9) {
+      best = cost;
+      best_k = kc;
+    }
+  }
+  return best_k;
 }
 
 int visc_ctas(const ViscArgs& a) {
