@@ -73,7 +73,7 @@ struct cbns_ctx {
   // hybrid flux: the learned sensor's parameters and per-face decisions
   float* sensor_params = nullptr;  // device, CBNS_SENSOR_NPARAM floats
   unsigned char* mask = nullptr;   // device, one byte per face: the decisions the fluxes use
-  unsigned char* mask_raw = nullptr;  // device: the network's decisions before widening
+  unsigned* bits[2] = {nullptr, nullptr};  // device: the network's decisions as bits, and widened along i and j
   float* wflux = nullptr;  // device, 8 floats per face: WENO5 fluxes of the stage's WENO5 faces
   int2* wlist = nullptr;   // device, up to one entry per face: the step's WENO5 faces
   long nfaces = 0;
@@ -429,9 +429,8 @@ void drop_graph(cbns_ctx* c) {
 // batched launches of a batch).
 struct SensorSet {
   MaskArgs m;
-  DilateArgs w[3];  // widening in i, j, k: raw -> mask -> raw -> mask
+  DilateArgs w;  // widening: bits -> bits -> mask and list
   AuditArgs au;
-  ListArgs li;
 };
 
 SensorSet sensor_set(cbns_ctx* c, const double* q, bool check_done, bool every_step, unsigned widen, bool hold) {
@@ -447,44 +446,33 @@ SensorSet sensor_set(cbns_ctx* c, const double* q, bool check_done, bool every_s
   m.params = c->sensor_params;
   m.tau = c->sensor_tau;
   m.every = every;
-  m.mask = c->mask_raw;
+  m.bits = c->bits[0];
   m.st = c->st;
   m.check_done = check_done;
-  unsigned char* bufs[4] = {c->mask_raw, c->mask, c->mask_raw, c->mask};
-  for (int dim = 0; dim < 3; ++dim) {
-    DilateArgs& w = ss.w[dim];
-    w.d = c->d;
-    w.in = bufs[dim];
-    w.out = bufs[dim + 1];
-    w.dim = dim;
-    w.along = 1 + (int)wn;
-    w.across = (int)wn;
-    w.st = c->st;
-    w.count = dim == 2;
-    w.every = every;
-    w.hold = hold;
-    w.check_done = check_done;
-  }
+  DilateArgs& w = ss.w;
+  w.d = c->d;
+  w.in = c->bits[0];
+  w.mid = c->bits[1];
+  w.out = c->mask;
+  w.list = c->wlist;
+  w.along = 1 + (int)wn;
+  w.across = (int)wn;
+  w.st = c->st;
+  w.every = every;
+  w.hold = hold;
+  w.check_done = check_done;
   AuditArgs& a = ss.au;
   a.d = c->d;
   a.gamma = (float)c->ph.gamma;
   a.gam1 = (float)c->ph.gam1;
   a.gam1_inv = (float)c->ph.gam1_inv;
-  a.q = q;
+  a.q = copy32(c, q);
   for (int k = 0; k < 10; ++k) a.area[k] = c->f.area[k];
   a.mask = c->mask;
   a.stride = c->audit_stride;
   a.bound = c->audit_bound;
   a.st = c->st;
   a.check_done = check_done;
-  ListArgs& l = ss.li;
-  l.d = c->d;
-  l.mask = c->mask;
-  l.nf = c->nfaces;
-  l.st = c->st;
-  l.list = c->wlist;
-  l.check_done = check_done;
-  l.every = every;
   return ss;
 }
 
@@ -506,8 +494,8 @@ int sensor_launch(cbns_ctx* c, const double* q, bool check_done, bool every_step
       n += 2;
     }
     // widening (held: the count only)
-    for (int dim = hold ? 2 : 0; dim < 3; ++dim) {
-      CK(launch_sensor_dilate(ss.w[dim], c->stream));
+    for (int pass = hold ? 1 : 0; pass < 2; ++pass) {
+      CK(launch_sensor_dilate(ss.w, pass, c->stream));
       n += 1;
     }
   }
@@ -516,12 +504,7 @@ int sensor_launch(cbns_ctx* c, const double* q, bool check_done, bool every_step
     CK(launch_sensor_audit(ss.au, c->stream));
   }
   n += 1;
-  if (!hold) {
-    Prof p(c, PK_WENO);
-    CK(launch_weno_list(c->d, c->mask, c->nfaces, c->st, c->wlist, check_done, ss.m.every, c->stream));
-    n += 1;
-  }
-  c->launches += n;  // sensor sweeps, widening passes, the audit, the WENO5-face list
+  c->launches += n;  // sensor sweeps, widening passes, the audit
   return CBNS_OK;
 }
 
@@ -620,8 +603,8 @@ struct cbns_batch {
   cudaStream_t stream = nullptr;           // the caller's, or owned by the batch
   bool own_stream = false;
   std::vector<cudaStream_t> saved;         // the blocks' streams before the batch
-  // the blocks' own kernels (the sensor sweeps, widening, audit and WENO5-face
-  // lists; boundary and viscous kernels unless every block is far field) are
+  // the blocks' own kernels (the sensor sweeps, widening and audit, the WENO5-face
+  // passes; boundary and viscous kernels unless every block is far field) are
   // captured on side streams, so the graph runs different blocks' small
   // kernels side by side between the batched launches
   std::vector<cudaStream_t> side;
@@ -648,18 +631,16 @@ struct cbns_batch {
   int* div_cta = nullptr;            // nblocks + 1 (the divergence kernel's CTAs)
   int bc_total = 0, visc_total = 0, div_total = 0;
   // hybrid, every block with the same network: the sensor sweeps, widening
-  // passes, audits and WENO5-face lists of all blocks in one launch each
+  // passes and audits of all blocks in one launch each
   bool sensor_batched = false;
   void* stables = nullptr;           // one allocation holding the tables below
   MaskArgs* mask_tab = nullptr;      // nblocks
-  DilateArgs* dil_tab = nullptr;     // 3 passes x nblocks
+  DilateArgs* dil_tab = nullptr;     // nblocks
   AuditArgs* aud_tab = nullptr;      // nblocks
-  ListArgs* list_tab = nullptr;      // nblocks
-  int* dil_cta = nullptr;            // 3 passes x (nblocks + 1)
+  int* dil_cta = nullptr;            // nblocks + 1 (either pass)
   int* aud_cta = nullptr;            // nblocks + 1
-  int* list_cta = nullptr;           // nblocks + 1
   long* ipre = nullptr;              // 2 x (nblocks + 1): sweep work items of the two kinds
-  int dil_total[3] = {0, 0, 0}, aud_total = 0, list_total = 0;
+  int dil_total = 0, aud_total = 0;
   long items_total[2] = {0, 0};
   std::vector<int> roles;     // (lq, lp, ls) per block at capture
   std::vector<unsigned long long> gens;  // the blocks' graph_gen at capture
@@ -702,55 +683,45 @@ int batch_sensor_tables(cbns_batch* b) {
   }
   if (!b->stables) {
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t o1 = up(nb * sizeof(MaskArgs)), o2 = o1 + up(3 * nb * sizeof(DilateArgs)),
-                 o3 = o2 + up(nb * sizeof(AuditArgs)), o4 = o3 + up(nb * sizeof(ListArgs)),
-                 o5 = o4 + up(3 * (nb + 1) * sizeof(int)), o6 = o5 + up((nb + 1) * sizeof(int)),
-                 o7 = o6 + up((nb + 1) * sizeof(int)), o8 = o7 + up(2 * (nb + 1) * sizeof(long));
-    CK(cudaMalloc(&b->stables, o8));
+    const size_t o1 = up(nb * sizeof(MaskArgs)), o2 = o1 + up(nb * sizeof(DilateArgs)),
+                 o3 = o2 + up(nb * sizeof(AuditArgs)), o4 = o3 + up((nb + 1) * sizeof(int)),
+                 o5 = o4 + up((nb + 1) * sizeof(int)), o6 = o5 + up(2 * (nb + 1) * sizeof(long));
+    CK(cudaMalloc(&b->stables, o6));
     char* t = static_cast<char*>(b->stables);
     b->mask_tab = reinterpret_cast<MaskArgs*>(t);
     b->dil_tab = reinterpret_cast<DilateArgs*>(t + o1);
     b->aud_tab = reinterpret_cast<AuditArgs*>(t + o2);
-    b->list_tab = reinterpret_cast<ListArgs*>(t + o3);
-    b->dil_cta = reinterpret_cast<int*>(t + o4);
-    b->aud_cta = reinterpret_cast<int*>(t + o5);
-    b->list_cta = reinterpret_cast<int*>(t + o6);
-    b->ipre = reinterpret_cast<long*>(t + o7);
+    b->dil_cta = reinterpret_cast<int*>(t + o3);
+    b->aud_cta = reinterpret_cast<int*>(t + o4);
+    b->ipre = reinterpret_cast<long*>(t + o5);
   }
   std::vector<MaskArgs> mt(nb);
-  std::vector<DilateArgs> dt(3 * nb);
+  std::vector<DilateArgs> dt(nb);
   std::vector<AuditArgs> at(nb);
-  std::vector<ListArgs> lt(nb);
-  std::vector<int> dc(3 * (nb + 1), 0), ac(nb + 1, 0), lc(nb + 1, 0);
+  std::vector<int> dc(nb + 1, 0), ac(nb + 1, 0);
   std::vector<long> ip(2 * (nb + 1), 0);
   for (int i = 0; i < nb; ++i) {
     cbns_ctx* c = b->blk[i];
     const SensorSet ss = sensor_set(c, c->qb[c->lq], true, false, 0, false);
     mt[i] = ss.m;
-    for (int dim = 0; dim < 3; ++dim) dt[dim * nb + i] = ss.w[dim];
+    dt[i] = ss.w;
     at[i] = ss.au;
-    lt[i] = ss.li;
-    for (int dim = 0; dim < 3; ++dim)
-      dc[dim * (nb + 1) + i + 1] = dc[dim * (nb + 1) + i] + sensor_dilate_ctas(c->d, dim);
+    dc[i + 1] = dc[i] + sensor_dilate_ctas(c->d);
     ac[i + 1] = ac[i] + sensor_audit_ctas(ss.au);
-    lc[i + 1] = lc[i] + weno_list_ctas(c->d);
     long n0, n1;
     sensor_mask_items(c->d, &n0, &n1);
     ip[i + 1] = ip[i] + n0;
     ip[nb + 1 + i + 1] = ip[nb + 1 + i] + n1;
   }
-  for (int dim = 0; dim < 3; ++dim) b->dil_total[dim] = dc[dim * (nb + 1) + nb];
+  b->dil_total = dc[nb];
   b->aud_total = ac[nb];
-  b->list_total = lc[nb];
   b->items_total[0] = ip[nb];
   b->items_total[1] = ip[2 * nb + 1];
   CK(cudaMemcpyAsync(b->mask_tab, mt.data(), nb * sizeof(MaskArgs), cudaMemcpyHostToDevice, b->stream));
-  CK(cudaMemcpyAsync(b->dil_tab, dt.data(), 3 * nb * sizeof(DilateArgs), cudaMemcpyHostToDevice, b->stream));
+  CK(cudaMemcpyAsync(b->dil_tab, dt.data(), nb * sizeof(DilateArgs), cudaMemcpyHostToDevice, b->stream));
   CK(cudaMemcpyAsync(b->aud_tab, at.data(), nb * sizeof(AuditArgs), cudaMemcpyHostToDevice, b->stream));
-  CK(cudaMemcpyAsync(b->list_tab, lt.data(), nb * sizeof(ListArgs), cudaMemcpyHostToDevice, b->stream));
-  CK(cudaMemcpyAsync(b->dil_cta, dc.data(), 3 * (nb + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+  CK(cudaMemcpyAsync(b->dil_cta, dc.data(), (nb + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   CK(cudaMemcpyAsync(b->aud_cta, ac.data(), (nb + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-  CK(cudaMemcpyAsync(b->list_cta, lc.data(), (nb + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   CK(cudaMemcpyAsync(b->ipre, ip.data(), 2 * (nb + 1) * sizeof(long), cudaMemcpyHostToDevice, b->stream));
   b->sensor_batched = true;
   return CBNS_OK;
@@ -865,15 +836,13 @@ int batch_enqueue_body(cbns_batch* b) {
   b->blk[0]->launches += 1;
   bool forked = false;
   if (b->hyb && b->sensor_batched) {
-    // every block's decisions: sweeps, widening, audit, WENO5-face list
+    // every block's decisions: sweeps, widening, audit
     CK(launch_sensor_mask_batched(b->mask_tab, b->ipre, b->ipre + nb + 1, b->items_total[0], b->items_total[1], nb,
                                   b->stream));
-    for (int dim = 0; dim < 3; ++dim)
-      CK(launch_sensor_dilate_batched(b->dil_tab + dim * nb, b->dil_cta + dim * (nb + 1), nb, b->dil_total[dim],
-                                      b->stream));
+    for (int pass = 0; pass < 2; ++pass)
+      CK(launch_sensor_dilate_batched(b->dil_tab, b->dil_cta, nb, b->dil_total, pass, b->stream));
     CK(launch_sensor_audit_batched(b->aud_tab, b->aud_cta, nb, b->aud_total, b->stream));
-    CK(launch_weno_list_batched(b->list_tab, b->list_cta, nb, b->list_total, b->stream));
-    b->blk[0]->launches += 8;
+    b->blk[0]->launches += 5;
   } else if (b->hyb) {
     RET(batch_fork(b));
     forked = true;
@@ -1120,8 +1089,10 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
     double* tmp = nullptr;
     rc = dalloc(c, &tmp, (size_t)(c->nfaces + 7) / 8);
     c->mask = reinterpret_cast<unsigned char*>(tmp);
-    if (rc == CBNS_OK) rc = dalloc(c, &tmp, (size_t)(c->nfaces + 7) / 8);
-    c->mask_raw = reinterpret_cast<unsigned char*>(tmp);
+    for (int b = 0; b < 2 && rc == CBNS_OK; ++b) {
+      rc = dalloc(c, &tmp, (size_t)(bit_words(d) + 1) / 2);
+      c->bits[b] = reinterpret_cast<unsigned*>(tmp);
+    }
     if (rc == CBNS_OK) rc = dalloc(c, &tmp, (size_t)c->nfaces * 4);
     c->wflux = reinterpret_cast<float*>(tmp);
     if (rc == CBNS_OK) rc = dalloc(c, &tmp, (size_t)c->nfaces);

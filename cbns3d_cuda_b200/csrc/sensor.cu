@@ -292,120 +292,136 @@ __global__ void zero_grad(float* G, float* loss) {
 }
 
 // ---------------------------------------------------------------- widening
-// Grid of one pass: x over the faces of a line along i (128 per CTA), y over
-// groups of lines along the walked direction, z over (face direction, the
-// third index).  Pass dim 0 and 1: the thread walks j (lines along j, groups
-// of DLJ), the CTA holds k; pass dim 2: the thread walks k (groups of DLK),
-// the CTA holds j.  So the widening of passes 1 and 2 runs along the thread's
-// own walk as a sliding window sum (two loads per face whatever the width),
-// and that of pass 0 along i from a line segment staged in shared memory with
-// its halo.  No index division per face.
-constexpr int DLJ = 16, DLK = 32;
-__host__ __device__ __forceinline__ dim3 dilate_grid(const Dims& d, int dim) {
-  const unsigned gx = (unsigned)((d.IM - 1 + 127) / 128);
-  if (dim == 2) return dim3(gx, (unsigned)((d.KM - 1 + DLK - 1) / DLK), (unsigned)(3 * (d.JM - 1)));
-  return dim3(gx, (unsigned)((d.JM - 1 + DLJ - 1) / DLJ), (unsigned)(3 * (d.KM - 1)));
+// Both passes take one 32-face word per thread, DT threads per CTA.  Three
+// passes of a load per face and window place on bytes, and one that listed the
+// faces from the bytes, took 207 + 55 us per network step on a 256x256x128
+// grid.  On bits 32 faces share every load and OR, and the words that pass 1
+// has in registers give the list: 18 + 37 us, the rest the 25 MB of bytes and
+// their 32 warp-wide stores per warp of words.
+constexpr int DT = 256;
+
+// the kind and the place (word of the line, line indices) of word w
+__device__ __forceinline__ BitRows bit_place(const Dims& d, long w, int& kind, int& x, int& j, int& k) {
+  BitRows b = bit_rows(d, 2);
+  kind = 2;
+  while (w < b.word) b = bit_rows(d, --kind);
+  const unsigned r = (unsigned)(w - b.word), line = r / (unsigned)b.W;
+  x = (int)(r - line * (unsigned)b.W);
+  k = (int)(line / (unsigned)b.n1);
+  j = (int)(line - (unsigned)k * (unsigned)b.n1);
+  return b;
 }
 
-// CTA (bx, by, bz) of one block's widening grid for pass a.dim
-__device__ __forceinline__ void dilate_body(const DilateArgs& a, unsigned bx, unsigned by, unsigned bz) {
+// pass 0 or 1 for the CTA bx of one block's grid
+template <int PASS>
+__device__ __forceinline__ void dilate_body(const DilateArgs& a, unsigned bx) {
   if (a.check_done && a.st->done) return;
-  const bool lead = bx == 0 && by == 0 && bz == 0 && threadIdx.x == 0;
+  const bool lead = bx == 0 && threadIdx.x == 0;
   if (a.hold || !sensor_step(a.st, a.every)) {
     // decisions of an earlier step: only the statistics, that step's count
-    if (a.count && lead) atomicAdd(&a.st->weno_faces, a.st->weno_last);
+    if (PASS == 1 && lead) atomicAdd(&a.st->weno_faces, a.st->weno_last);
     return;
   }
-  if (a.dim == 0 && lead) a.st->weno_last = 0;  // the last pass counts anew
+  if (PASS == 0 && lead) {  // pass 1 counts and lists anew
+    a.st->weno_last = 0;
+    for (int m = 0; m < 3; ++m) a.st->weno_listed[m] = 0;
+  }
   const Dims& d = a.d;
-  const int IM = d.IM, JM = d.JM, KM = d.KM;
-  const bool walk_k = a.dim == 2;
-  const int zc = walk_k ? JM - 1 : KM - 1;
-  const int dir = (int)bz / zc, fixed = (int)bz % zc;
-  // extents (n0, n1, n2) and first index of this direction's faces
-  const int n0 = dir == 0 ? IM - 1 : IM - 2, n1 = dir == 1 ? JM - 1 : JM - 2, n2 = dir == 2 ? KM - 1 : KM - 2;
-  const long first = dir == 0 ? 0
-                              : (dir == 1 ? (long)(IM - 1) * (JM - 2) * (KM - 2)
-                                          : (long)(IM - 1) * (JM - 2) * (KM - 2) + (long)(IM - 2) * (JM - 1) * (KM - 2));
-  if (fixed >= (walk_k ? n1 : n2)) return;  // uniform per CTA
-  const int x0 = (int)bx * 128 + (int)threadIdx.x;
-  const bool valid = x0 < n0;
-  // the thread's walk: positions q0 .. q1-1 along j (walk_k: along k), face
-  // index base + q * step
-  const int nq = walk_k ? n2 : n1, dl = walk_k ? DLK : DLJ;
-  const int q0 = (int)by * dl, q1 = min(nq, q0 + dl);
-  const long step = walk_k ? (long)n0 * n1 : (long)n0;
-  const long base = first + x0 + (walk_k ? (long)n0 * fixed : (long)n0 * n1 * fixed);
-  unsigned cnt = 0;
-  {
-    const unsigned char* __restrict__ in = a.in;
-    unsigned char* __restrict__ out = a.out;
-    const int w = a.dim == dir ? a.along : a.across;
-    if (a.dim == 0) {
-      // along i: each line's 128 faces and a halo of w either side staged in
-      // shared memory (coalesced), then each thread ORs its window there
-      constexpr int WMAX = 16;
-      __shared__ unsigned char row[128 + 2 * WMAX];
-      const int t = threadIdx.x;
-      const int xb = (int)bx * 128;  // first face of the CTA's segment
-      for (int q = q0; q < q1; ++q) {
-        const long e = base + q * step;  // this thread's face (x0 = xb + t)
-        unsigned dec = 0;
-        if (w <= WMAX) {
-          __syncthreads();  // the previous line's window reads are done
-          row[WMAX + t] = valid ? __ldg(in + e) : 0;
-          if (t < WMAX) {
-            const int xl = xb - WMAX + t, xr = xb + 128 + t;  // halo faces
-            row[t] = (xl >= 0 && xl < n0) ? __ldg(in + e - WMAX) : 0;
-            row[WMAX + 128 + t] = (xr < n0) ? __ldg(in + e + 128) : 0;
-          }
-          __syncthreads();
-          if (valid)
-            for (int o = -w; o <= w; ++o) dec |= row[WMAX + t + o];
-        } else if (valid) {
-          const int lo = max(-w, -x0), hi = min(w, n0 - 1 - x0);
-          for (int o = lo; o <= hi; ++o) dec |= __ldg(in + e + o);
-        }
-        if (valid) {
-          out[e] = (unsigned char)dec;
-          cnt += dec;
-        }
+  const long words = bit_words(d), w = (long)bx * DT + threadIdx.x;
+  int kind = 0, x = 0, j = 0, k = 0;
+  BitRows b{};
+  unsigned v = 0;
+  if (PASS == 0) {
+    if (w >= words) return;
+    b = bit_place(d, w, kind, x, j, k);
+    // OR of the lines j - wj .. j + wj, then of the faces x - wi .. x + wi of it
+    const int wi = kind == 0 ? a.along : a.across, wj = kind == 1 ? a.along : a.across;
+    unsigned prev = 0, cur = 0, next = 0;
+    const unsigned* p = a.in + b.word + (long)k * b.n1 * b.W + x;
+    for (int jj = max(0, j - wj); jj <= min(b.n1 - 1, j + wj); ++jj) {
+      const unsigned* q = p + (long)jj * b.W;
+      cur |= __ldg(q);
+      if (x > 0) prev |= __ldg(q - 1);
+      if (x + 1 < b.W) next |= __ldg(q + 1);
+    }
+    v = cur;
+    for (int s = 1; s <= wi; ++s) v |= __funnelshift_l(prev, cur, s) | __funnelshift_r(cur, next, s);
+    const int n = b.n0 - 32 * x;  // faces of the line's last word
+    if (n < 32) v &= (1u << n) - 1u;
+    a.mid[w] = v;
+  } else {
+    __shared__ int wcnt[3][DT / 32], base[3];
+    int e = 0, n = 0;
+    unsigned oa = 0;
+    if (w < words) {
+      b = bit_place(d, w, kind, x, j, k);
+      const int wk = kind == 2 ? a.along : a.across;
+      const long plane = (long)b.n1 * b.W;
+      const unsigned* p = a.mid + w;
+      for (int kk = max(0, k - wk); kk <= min(b.n2 - 1, k + wk); ++kk) v |= __ldg(p + (kk - k) * plane);
+      e = (int)(b.face + ((long)k * b.n1 + j) * b.n0 + 32 * x);
+      n = min(32, b.n0 - 32 * x);
+      oa = (unsigned)node_off(d, 32 * x + (kind != 0), j + (kind != 1), k + (kind != 2));  // low node of the word's first face
+    }
+    // where each word's faces go in its kind's list: a scan over the warp, then
+    // over the CTA's warps, and one atomic per kind that the CTA meets
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int pos = 0;
+    for (int m = 0; m < 3; ++m) {
+      const int c = kind == m ? __popc(v) : 0;
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
-    } else if (valid) {
-      // along the walk: a sliding window sum of the 0/1 decisions
-      int sum = 0;
-      for (int q = max(0, q0 - w); q <= min(nq - 1, q0 + w); ++q) sum += __ldg(in + base + q * step);
-      for (int q = q0; q < q1; ++q) {
-        const unsigned dec = sum > 0 ? 1u : 0u;
-        out[base + q * step] = (unsigned char)dec;
-        cnt += dec;
-        if (q - w >= 0) sum -= __ldg(in + base + (q - w) * step);
-        if (q + 1 + w < nq) sum += __ldg(in + base + (q + 1 + w) * step);
+      if (kind == m) pos = incl - c;
+      if (lane == 31) wcnt[m][warp] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+      const int m = threadIdx.x;
+      int tot = 0;
+      for (int q = 0; q < DT / 32; ++q) {
+        const int c = wcnt[m][q];
+        wcnt[m][q] = tot;
+        tot += c;
+      }
+      if (tot) {
+        base[m] = (int)bit_rows(d, m).face + (int)atomicAdd(&a.st->weno_listed[m], (unsigned)tot);
+        atomicAdd(&a.st->weno_faces, (unsigned long long)tot);
+        atomicAdd(&a.st->weno_last, (unsigned long long)tot);
       }
     }
-  }
-  if (a.count) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) {
-      atomicAdd(&a.st->weno_faces, (unsigned long long)cnt);
-      atomicAdd(&a.st->weno_last, (unsigned long long)cnt);
+    __syncthreads();
+    pos += base[kind] + wcnt[kind][warp];
+    // each lane's word as 32 bytes and its list entries, the warp on one word
+    // at a time
+    for (int s = 0; s < 32; ++s) {
+      const int ns = __shfl_sync(0xffffffffu, n, s), es = __shfl_sync(0xffffffffu, e, s);
+      const unsigned vs = __shfl_sync(0xffffffffu, v, s);
+      const bool on = (vs >> lane) & 1u;
+      if (lane < ns) a.out[es + lane] = on;
+      if (vs) {
+        const int ps = __shfl_sync(0xffffffffu, pos, s), ks = __shfl_sync(0xffffffffu, kind, s);
+        const unsigned os = __shfl_sync(0xffffffffu, oa, s);
+        if (on) a.list[ps + __popc(vs & ((1u << lane) - 1u))] = list_entry(es + lane, ks, os + lane);
+      }
     }
   }
 }
 
-__global__ void __launch_bounds__(128) sensor_dilate_kernel(const DilateArgs a) {
-  dilate_body(a, blockIdx.x, blockIdx.y, blockIdx.z);
+template <int PASS>
+__global__ void __launch_bounds__(DT) sensor_dilate_kernel(const DilateArgs a) {
+  dilate_body<PASS>(a, blockIdx.x);
 }
 
 // Many blocks in one launch: block b owns CTAs cta[b] .. cta[b+1]-1, args[b]
-// are its DilateArgs (all of one pass).
-__global__ void __launch_bounds__(128) sensor_dilate_batched(const DilateArgs* args, const int* cta, int nblocks) {
+// are its DilateArgs.
+template <int PASS>
+__global__ void __launch_bounds__(DT) sensor_dilate_batched(const DilateArgs* args, const int* cta, int nblocks) {
   const int b = block_of_cta(cta, nblocks, (int)blockIdx.x);
-  const DilateArgs& a = args[b];
-  const dim3 g = dilate_grid(a.d, a.dim);
-  const unsigned l = blockIdx.x - (unsigned)__ldg(cta + b);
-  dilate_body(a, l % g.x, (l / g.x) % g.y, l / (g.x * g.y));
+  dilate_body<PASS>(args[b], blockIdx.x - (unsigned)__ldg(cta + b));
 }
 
 // ---------------------------------------------------------------- audit
@@ -423,7 +439,7 @@ __device__ __forceinline__ void audit_body(const AuditArgs& a, unsigned bx) {
   if (e < nf && a.mask[e] == 0 && decode_face(d, e, dir, i, j, k)) {
     const long sd = dir == 0 ? 1 : (dir == 1 ? d.PX : d.PL);
     const long oa = node_off(d, i, j, k), ob = oa + sd;
-    auto ld = [&](int p, int n) -> float { return (float)__ldg(a.q + n * d.VOL + oa + (p - 2) * sd); };
+    auto ld = [&](int p, int n) -> float { return __ldg(a.q + n * d.VOL + oa + (p - 2) * sd); };
     const float nx = (float)(0.5 * (__ldg(a.area[3 * dir] + oa) + __ldg(a.area[3 * dir] + ob)));
     const float ny = (float)(0.5 * (__ldg(a.area[3 * dir + 1] + oa) + __ldg(a.area[3 * dir + 1] + ob)));
     const float nz = (float)(0.5 * (__ldg(a.area[3 * dir + 2] + oa) + __ldg(a.area[3 * dir + 2] + ob)));
@@ -441,14 +457,18 @@ __device__ __forceinline__ void audit_body(const AuditArgs& a, unsigned bx) {
     if (!(err == err)) err = 3.0e38f;
     audited = true;
   }
-  const unsigned full = 0xffffffffu;
-  const unsigned n_aud = __popc(__ballot_sync(full, audited));
+  // one set of atomics per CTA, the maximum's only where it grows
+  __shared__ float wmax[4];
   float m = err;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(full, m, o));
-  if ((threadIdx.x & 31) == 0 && n_aud) {
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+  const int n_aud = __syncthreads_count(audited);
+  if (threadIdx.x == 0 && n_aud) {
+    m = fmaxf(fmaxf(wmax[0], wmax[1]), fmaxf(wmax[2], wmax[3]));
     atomicAdd(&a.st->audit_faces, (unsigned long long)n_aud);
-    atomicMax(reinterpret_cast<int*>(&a.st->audit_max), __float_as_int(m));  // m >= 0: int order = float order
+    if (m > *(volatile float*)&a.st->audit_max)
+      atomicMax(reinterpret_cast<int*>(&a.st->audit_max), __float_as_int(m));  // m >= 0: int order = float order
     if (m > a.bound && atomicExch(&a.st->force_weno, 1) == 0) atomicAdd(&a.st->audit_fail_steps, 1u);
   }
 }
@@ -506,13 +526,12 @@ cudaError_t launch_sensor_audit(const AuditArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-int sensor_dilate_ctas(const Dims& d, int dim) {
-  const dim3 g = dilate_grid(d, dim);
-  return (int)(g.x * g.y * g.z);
-}
+int sensor_dilate_ctas(const Dims& d) { return (int)((bit_words(d) + DT - 1) / DT); }
 
-cudaError_t launch_sensor_dilate(const DilateArgs& a, cudaStream_t s) {
-  sensor_dilate_kernel<<<dilate_grid(a.d, a.dim), 128, 0, s>>>(a);
+cudaError_t launch_sensor_dilate(const DilateArgs& a, int pass, cudaStream_t s) {
+  const int ctas = sensor_dilate_ctas(a.d);
+  if (pass == 0) sensor_dilate_kernel<0><<<ctas, DT, 0, s>>>(a);
+  else sensor_dilate_kernel<1><<<ctas, DT, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -523,10 +542,11 @@ cudaError_t launch_sensor_audit_batched(const AuditArgs* args, const int* cta, i
   return cudaGetLastError();
 }
 
-cudaError_t launch_sensor_dilate_batched(const DilateArgs* args, const int* cta, int nblocks, int total,
+cudaError_t launch_sensor_dilate_batched(const DilateArgs* args, const int* cta, int nblocks, int total, int pass,
                                          cudaStream_t s) {
   if (total <= 0) return cudaSuccess;
-  sensor_dilate_batched<<<total, 128, 0, s>>>(args, cta, nblocks);
+  if (pass == 0) sensor_dilate_batched<0><<<total, DT, 0, s>>>(args, cta, nblocks);
+  else sensor_dilate_batched<1><<<total, DT, 0, s>>>(args, cta, nblocks);
   return cudaGetLastError();
 }
 

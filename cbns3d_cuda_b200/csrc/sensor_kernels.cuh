@@ -20,8 +20,34 @@ struct SampleArgs {
   unsigned* count;          // device counter, incremented per sampled face
 };
 
+// The network's decisions before widening, one bit per face: each line of faces
+// along i starts a word (W words a line, bit x & 31 of word x >> 5 for face x),
+// the lines of each kind in the order of the global face index, the kinds one
+// after the other.
+struct BitRows {
+  int n0, n1, n2, W;  // faces along i, lines along the two other directions, words per line
+  long face, word;    // the kind's first face index and first word
+};
+__host__ __device__ inline BitRows bit_rows(const Dims& d, int kind) {
+  BitRows b{d.IM - 1, d.JM - 2, d.KM - 2, 0, 0, 0};
+  b.W = (b.n0 + 31) / 32;
+  for (int k = 1; k <= kind; ++k) {
+    b.face += (long)b.n0 * b.n1 * b.n2;
+    b.word += (long)b.W * b.n1 * b.n2;
+    b.n0 = d.IM - 2;
+    b.n1 = k == 1 ? d.JM - 1 : d.JM - 2;
+    b.n2 = k == 2 ? d.KM - 1 : d.KM - 2;
+    b.W = (b.n0 + 31) / 32;
+  }
+  return b;
+}
+__host__ __device__ inline long bit_words(const Dims& d) {
+  const BitRows b = bit_rows(d, 2);
+  return b.word + (long)b.W * b.n1 * b.n2;
+}
+
 // Per-step decision of the hybrid flux: features of every face of q, the
-// network on the tensor cores, mask[e] = 1 (WENO5) where p >= tau else 0.
+// network on the tensor cores, bit 1 (WENO5) where p >= tau else 0.
 struct MaskArgs {
   Dims d;
   float gamma, gam1;
@@ -30,7 +56,7 @@ struct MaskArgs {
   const float* params;      // CBNS_SENSOR_NPARAM floats (device)
   float tau;
   unsigned every;           // evaluate on steps with steps % every == 1 % every (1: always)
-  unsigned char* mask;      // one byte per face
+  unsigned* bits;           // one bit per face, before widening (BitRows)
   StepState* st;            // statistics, failure flag, done flag
   int check_done;
 };
@@ -42,21 +68,31 @@ struct MaskArgs {
 // it reaches at most one more node of the 6-node stencils near it, and a
 // curved front (a blast) reaches grid lines next to those it crossed at the
 // step's start, so those faces stay on WENO5 for the step's three stages.
-// Three separable passes (one per index direction); the last one counts the
-// WENO5 faces.  When the network runs only every n-th step, its decisions
-// must hold for n steps: widths 1 + n along and n across.
+// The OR over the window is separable: a pass along i and j on the decision
+// bits (pass 0), a pass along k that writes the decision bytes and counts and
+// lists the WENO5 faces (pass 1), each kind in its own list of
+// st->weno_listed[kind] entries that starts at the kind's first face index.
+// When the network runs only every n-th step, its
+// decisions must hold for n steps: widths 1 + n along and n across.
 struct DilateArgs {
   Dims d;
-  const unsigned char* in;
-  unsigned char* out;
-  int dim;                 // index direction of this pass: 0 = i, 1 = j, 2 = k
-  int along, across;       // widening widths (faces)
-  StepState* st;           // WENO5 faces are counted when count != 0
-  int count;
+  const unsigned* in;      // decision bits
+  unsigned* mid;           // after pass 0
+  unsigned char* out;      // one byte per face
+  int2* list;              // the WENO5 faces (list_entry)
+  int along, across;       // widening widths (faces, below 32)
+  StepState* st;
   unsigned every;          // as MaskArgs::every; the count is kept every step
   int hold;                // the decisions hold this step: count only (per-call path)
   int check_done;
 };
+
+// A list entry: the face index and, packed, its kind (0 i-, 1 j-, 2 k-face,
+// bits 30-31) and the node offset of its low node (bits 0-29; contexts of the
+// hybrid precision keep VOL below 2^30).
+__device__ __forceinline__ int2 list_entry(int e, int kind, unsigned oa) {
+  return make_int2(e, (int)(((unsigned)kind << 30) | oa));
+}
 
 // true when the sensor is evaluated in the current step (steps counts from 1)
 __device__ __forceinline__ bool sensor_step(const StepState* st, unsigned every) {
@@ -70,7 +106,7 @@ __device__ __forceinline__ bool sensor_step(const StepState* st, unsigned every)
 struct AuditArgs {
   Dims d;
   float gamma, gam1, gam1_inv;
-  const double* q;
+  const float* q;  // the state's FP32 copy
   const double* area[10];
   const unsigned char* mask;
   unsigned stride;
@@ -82,16 +118,16 @@ struct AuditArgs {
 cudaError_t launch_sample_faces(const SampleArgs& a, cudaStream_t s);
 cudaError_t launch_sensor_mask(const MaskArgs& a, cudaStream_t s);
 cudaError_t launch_sensor_audit(const AuditArgs& a, cudaStream_t s);
-cudaError_t launch_sensor_dilate(const DilateArgs& a, cudaStream_t s);
+cudaError_t launch_sensor_dilate(const DilateArgs& a, int pass, cudaStream_t s);
 // Batched forms (many blocks in one launch): args and cta are device tables,
 // block b owning CTAs cta[b] .. cta[b+1]-1 of total, cta[b+1] - cta[b] the
 // block's count below.  Mask: ipre[b] .. ipre[b+1]-1 are block b's work items
 // of each kind (sensor_mask_items); every block's MaskArgs::params must hold
 // the same network (it is loaded once per CTA, from args[0]).
-int sensor_dilate_ctas(const Dims& d, int dim);  // pass dim's grid
+int sensor_dilate_ctas(const Dims& d);
 int sensor_audit_ctas(const AuditArgs& a);
 void sensor_mask_items(const Dims& d, long* items0, long* items1);
-cudaError_t launch_sensor_dilate_batched(const DilateArgs* args, const int* cta, int nblocks, int total,
+cudaError_t launch_sensor_dilate_batched(const DilateArgs* args, const int* cta, int nblocks, int total, int pass,
                                          cudaStream_t s);
 cudaError_t launch_sensor_audit_batched(const AuditArgs* args, const int* cta, int nblocks, int total,
                                         cudaStream_t s);

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(128) mlp_predict_tc_kernel(const float* __rest
 // So each node's primitives are formed once per direction, and a tile's
 // loads are coalesced along i.  A tile whose faces all have flat stencils is
 // decided linear at once; any other tile goes through the network on the
-// tensor cores and each thread writes the decision byte of its face.
+// tensor cores and each warp writes its 32 decisions as one word.
 constexpr int SW_T = 128;  // faces per tile = threads per CTA
 constexpr int SW_CH = 30;  // tiles per work item (a multiple of the 6-face window rotation)
 
@@ -87,27 +87,29 @@ struct SweepCtx {
   tc::Smem* s;
   unsigned phase;
   float zcut;
-  unsigned char* mask;
+  unsigned* bits;
 };
 
-// Decision of the thread's face e (when valid) from its features f; false if
-// a tensor-core wait timed out.  Called by all threads of the CTA.
-__device__ __forceinline__ bool classify(SweepCtx& c, int t, const float f[SN_IN], bool valid, long e) {
-  unsigned char dec = 0;
+// Decisions of the CTA's 128 faces (of which valid ones exist) from their
+// features f into the four words from `word` on; false if a tensor-core wait
+// timed out.  Called by all threads of the CTA.
+__device__ __forceinline__ bool classify(SweepCtx& c, int t, const float f[SN_IN], bool valid, long word) {
+  bool dec = false;
   const bool flat = feature_l1(f) < SN_FLAT;  // false for NaN features
   if (!__syncthreads_and(!valid || flat)) {
     tc::put_features(*c.s, t, f);
     float z = 0.f;
     if (!tc::run_tile(*c.s, t, c.phase, &z)) return false;
     // non-finite features (e.g. a non-physical state) fall back to WENO5
-    dec = (!flat && (z >= c.zcut || !(z == z))) ? 1 : 0;
+    dec = !flat && (z >= c.zcut || !(z == z));
   }
-  if (valid) c.mask[e] = dec;
+  const unsigned w = __ballot_sync(0xffffffffu, valid && dec);
+  if ((t & 31) == 0 && valid) c.bits[word + (t >> 5)] = w;
   return true;
 }
 
 // One work item (KIND 0: i-face rows; KIND 1: j- or k-face window sweeps) of
-// the block a: its decisions into a.mask.  Called by all threads of the CTA;
+// the block a: its decisions into a.bits.  Called by all threads of the CTA;
 // false if a tensor-core wait timed out (the CTA then classifies nothing more).
 template <int KIND>
 __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx& cx, RowSmem& rs, WinSmem& ws, int t) {
@@ -200,7 +202,7 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
 #pragma unroll
         for (int m = 0; m < SN_IN; ++m) f[m] = 0.f;
       }
-      ok = classify(cx, t, f, valid, i + (long)(IM - 1) * ((j - 1) + (long)(JM - 2) * (k - 1)));
+      ok = classify(cx, t, f, valid, (long)r * ((IM - 1 + 31) / 32) + seg * (SW_T / 32));
     }
   } else {  // j- or k-faces: a window sweep along the direction
     const bool dj = item < n0 + n1;
@@ -216,11 +218,12 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
     const bool valid = i <= IM - 2;
     const long sd = dj ? d.PX : d.PL;
     const int am = dj ? 3 : 6;  // J grad(eta) or J grad(zeta)
-    // offset of the sweep's position 0 for this column; face fc has global
-    // index e0 + fc * es
+    // offset of the sweep's position 0 for this column; face fc's line of
+    // decision bits starts at word line0 + fc * wstep
     const long obase = dj ? node_off(d, valid ? i : 1, 0, c) : node_off(d, valid ? i : 1, c, 0);
-    const long e0 = dj ? nfi + (i - 1) + (long)(IM - 2) * (JM - 1) * (c - 1) : nfi + nfj + (i - 1) + (long)(IM - 2) * (c - 1);
-    const long es = dj ? (long)(IM - 2) : (long)(IM - 2) * (JM - 2);
+    const BitRows br = bit_rows(d, dj ? 1 : 2);
+    const long line0 = br.word + (long)br.W * (dj ? (long)(JM - 1) * (c - 1) : c - 1) + seg * (SW_T / 32);
+    const long wstep = dj ? br.W : (long)br.W * (JM - 2);
     NodePrim W0, W1, W2, W3, W4, W5;
     float Aa[3], Ab[3];
     // step u (face f0+u) consumes node f0+3+u and the area vector of node f0+1+u
@@ -278,7 +281,7 @@ __device__ __forceinline__ bool mask_item(const MaskArgs& a, long item, SweepCtx
 #pragma unroll
         for (int m = 0; m < SN_IN; ++m) f[m] = 0.f;
       }
-      return classify(cx, t, f, valid, e0 + fc * es);
+      return classify(cx, t, f, valid, line0 + fc * wstep);
     };
     for (int fc = f0; ok && fc < f1; fc += 6) {
       ok = face(fc, W0, W1, W2, W3, W4, W5, Aa, Ab);
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(SW_T, 5) sensor_mask_kernel(const MaskArgs a) 
   if ((a.check_done && a.st->done) || !sensor_step(a.st, a.every)) return;
   const int t = threadIdx.x;
   const MaskSmem m = mask_setup(a.params, t);
-  SweepCtx cx{m.s, 0u, logit_cut(a.tau), a.mask};
+  SweepCtx cx{m.s, 0u, logit_cut(a.tau), a.bits};
   long it0, it1;
   mask_items(a.d, KIND, &it0, &it1);
   bool ok = true;
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(SW_T, 5) sensor_mask_batched(const MaskArgs* a
     if ((a.check_done && a.st->done) || !sensor_step(a.st, a.every)) continue;
     if (ok) {
       cx.zcut = logit_cut(a.tau);
-      cx.mask = a.mask;
+      cx.bits = a.bits;
       long it0, it1;
       mask_items(a.d, KIND, &it0, &it1);
       ok = mask_item<KIND>(a, it0 + (g - ipre[b]), cx, *m.rs, *m.ws, t);

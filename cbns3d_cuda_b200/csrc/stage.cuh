@@ -73,30 +73,12 @@ int stage_variants(bool fp32, bool hybrid);
 void stage32_prepare();
 cudaError_t launch_stage32(const StageArgs& a, int mode, bool visc, int variant, cudaStream_t s);
 cudaError_t launch_stage32_batched(const BatchStage& b, int mode, bool visc, bool hybrid, cudaStream_t s);
-// Hybrid: list the faces whose decision byte is set (once per step, after the
-// decisions are final; each face kind in its own list, st->weno_listed[kind]
-// receiving its length) ...
-cudaError_t launch_weno_list(const Dims& d, const unsigned char* mask, long nfaces, StepState* st, int2* list,
-                             bool check_done, unsigned every, cudaStream_t s);
-// ... and evaluate the listed faces (every face while force_weno is set) into
-// a.wflux, where the stage kernel reads them: before each hybrid stage-kernel
-// launch, on the same input.
+// Hybrid: evaluate the listed faces (the widening pass's lists; every face
+// while force_weno is set) into a.wflux, where the stage kernel reads them:
+// before each hybrid stage-kernel launch, on the same input.
 cudaError_t launch_weno_faces(const StageArgs& a, int mode, long nfaces, const int2* list, cudaStream_t s);
 // Size the evaluation kernel's grid (once, outside any stream capture).
 cudaError_t weno_prepare();
-// The lists of many blocks in one launch (after zeroing each block's count):
-// block b owns CTAs cta[b] .. cta[b+1]-1 of total, weno_list_ctas(its Dims) of them.
-struct ListArgs {
-  Dims d;
-  const unsigned char* mask;
-  long nf;
-  StepState* st;
-  int2* list;
-  int check_done;
-  unsigned every;  // the network's interval (MaskArgs::every): the lists are rebuilt on its steps only
-};
-int weno_list_ctas(const Dims& d);
-cudaError_t launch_weno_list_batched(const ListArgs* args, const int* cta, int nblocks, int total, cudaStream_t s);
 // modes 1..3 only; hybrid: the StageArgs carry decision masks.
 cudaError_t launch_stage_batched(const BatchStage& b, int mode, bool visc, bool fp32, bool hybrid, cudaStream_t s);
 constexpr int STAGE_TI = 16, STAGE_TJ = 15;  // columns of a CTA's tile
