@@ -1175,10 +1175,10 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   }
   // until cbns_autotune says otherwise, the variants and chunks it picks on
   // B200 for grids of a few million nodes: FP64 stages by TMA (about 10%
-  // faster than the synchronous variant) and the split precision runs 2 CTAs
-  // per SM, both with about 9 waves of CTAs; the hybrid runs 3 per SM (8%
-  // faster than 2) with chunks sized by the wave count and warm-up.  Where
-  // that makes fewer than four waves, the chunk of kchunk_small.
+  // faster than the synchronous variant) with about 9 waves of CTAs, the FP32
+  // kernels run 3 CTAs per SM (8% faster than 2) with chunks sized by the wave
+  // count and warm-up.  Where that makes fewer than four waves, the chunk of
+  // kchunk_small.
   const int per_sm = fp32 ? 3 : 2, slots = c->nsm * per_sm;
   c->stage_variant = 1;
   c->kchunk = fp32 ? kchunk_by_waves(ntiles, nint, slots, 0.5) : kchunk_for_waves(ntiles, nint, slots, 9.0);
@@ -1673,13 +1673,24 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
   RET(check_flux_ready(c));
   const bool fp32 = c->ph.precision != CBNS_PREC_FP64;
   const int nv = stage_variants(fp32, hybrid(c));
-  // time every variant on the current state (RHS-only mode: nothing is updated);
-  // the hybrid kernel is timed on the sensor's decisions for this state
+  // time every variant on the current state: an inviscid block's first stage
+  // into the spare buffer, whose interior holds nothing between steps (the
+  // RHS-only mode ranked the hybrid kernel's variants the other way: 2 CTAs per
+  // SM, whose three stages take 1.42 ms on a 256x256x128 block against 1.27
+  // for 3); a viscous block's stage writes its primitives, so there the
+  // RHS-only mode.  The hybrid kernel is timed on the sensor's decisions for
+  // this state
   if (hybrid(c)) {
     CK(cudaMemsetAsync(&c->st->force_weno, 0, sizeof(int), c->stream));
     RET(sensor_launch(c, c->qb[c->lq], false, true));
     c->percall_hold = 0;
   }
+  const int mode = c->ph.viscous ? 0 : 1;
+  double* const P0 = c->qb[c->lq];
+  int done = 0;  // a finished run's stages return at once: off while they are timed
+  CK(cudaMemcpyAsync(&done, &c->st->done, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemsetAsync(&c->st->done, 0, sizeof(int), c->stream));
+  RET(sync(c));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   if (cudaEventCreate(&e1) != cudaSuccess) {
@@ -1687,16 +1698,17 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
     g_last = "cudaEventCreate failed";
     return CBNS_ERR_CUDA;
   }
-  // the faster of two rounds of three RHS launches after one warm-up launch
+  // the faster of two rounds of three launches after one warm-up launch
   auto time_it = [&](int v, int kc, float* ms) -> int {
     c->stage_variant = v;
     c->kchunk = kc;
-    const StageArgs a = stage_args(c, c->qb[c->lq], nullptr, nullptr, c->staging, false);
-    RET(stage_launch(c, a, 0));
+    const StageArgs a = mode ? stage_args(c, P0, P0, P0, c->qb[c->ls], false)
+                             : stage_args(c, P0, nullptr, nullptr, c->staging, false);
+    RET(stage_launch(c, a, mode));
     *ms = 1e30f;
     for (int round = 0; round < 2; ++round) {
       CK(cudaEventRecord(e0, c->stream));
-      for (int r = 0; r < 3; ++r) RET(stage_launch(c, a, 0));
+      for (int r = 0; r < 3; ++r) RET(stage_launch(c, a, mode));
       CK(cudaEventRecord(e1, c->stream));
       CK(cudaEventSynchronize(e1));
       float t = 0.f;
@@ -1706,7 +1718,7 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
     return CBNS_OK;
   };
   // the context's current pair stays unless another is more than 1% faster:
-  // the candidates' RHS-only times differ by about that much where their full
+  // the candidates' single-launch times differ by about that much where their full
   // steps rank the other way
   const int v0 = c->stage_variant, kc0 = c->kchunk;
   int best = v0, best_kc = kc0, rc = CBNS_OK;
@@ -1728,6 +1740,8 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  CK(cudaMemcpyAsync(&c->st->done, &done, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  RET(sync(c));
   c->stage_variant = best;
   c->kchunk = best_kc;
   drop_graph(c);
