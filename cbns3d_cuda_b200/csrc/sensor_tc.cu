@@ -67,7 +67,7 @@ struct RowSmem {
 // The window sweeps stream each column's nodes through a per-thread ring of
 // SW_D slots filled by asynchronous copies (cp.async), SW_D faces ahead: slot
 // u % SW_D holds the 5 state values of node f0+3+u and the area vector of
-// node f0+1+u for face f0+u.  Two slots keep the sweep at 5 CTAs per SM (16
+// node f0+1+u for face f0+u.  Two slots keep the sweep at 5 CTAs per SM (8
 // KB of ring; four slots and 4 CTAs per SM measured 2% slower).
 constexpr int SW_D = 2;
 struct WinSmem {

@@ -384,10 +384,9 @@ int cbns_autotune(cbns_ctx* ctx, int* chosen);
 /* Use compiled variant `variant` of the stage kernel (0 .. count-1; count from
  * *count when not null, variant -1 only queries it).  FP64: 0 stages each
  * plane synchronously, 1 by TMA (the same arithmetic, to the rounding of a
- * separate compilation); FP32:
- * 2 + variant CTAs per SM.  A new context starts on variant 1 (FP64; hybrid
- * grids of at least two waves of 3-per-SM CTAs) or 0 (split, smaller hybrid
- * grids).  No counterpart in the reference. */
+ * separate compilation); FP32: 0 has the registers of 2 CTAs per SM, 1 of 3
+ * (the hybrid's 2 is accepted and runs 1's kernel).  A new context starts on
+ * variant 1.  No counterpart in the reference. */
 int cbns_stage_variant(cbns_ctx* ctx, int variant, int* count);
 /* Use k chunks of `kchunk` planes in the stage kernel's work items (one CTA
  * per tile and chunk; 1 .. KM-2, -1 only queries); *current (may be null)
