@@ -4,8 +4,9 @@
 // dt needs the largest FP64 spectral radius of the grid, and evaluating it at
 // every node (about 70 FP64 operations with four square roots) costs stage 3 a
 // tenth of its time.  Most nodes are far below the largest value already found,
-// so a node is evaluated in FP64 only if its FP32 bound reaches it; the maximum
-// is the same to the bit.
+// so a node is evaluated in FP64 only if its FP32 bound reaches it, or if its
+// squared sound speed is not safely positive in FP32 (the FP64 value may be a
+// NaN, which must end the run): the result is the same to the bit.
 #pragma once
 
 #include "cbns_common.cuh"
@@ -18,26 +19,36 @@ __device__ __forceinline__ F2 abs_(F2 x) {
   return each(x, [](float a) { return fabsf(a); });
 }
 
+__device__ __forceinline__ float min_(float x, float y) { return fminf(x, y); }
+__device__ __forceinline__ F2 min_(F2 x, F2 y) {
+  return each(x, y, [](float a, float b) { return fminf(a, b); });
+}
+
 // An upper bound of the spectral radius of a node (or two): q its state, A its
 // area vectors J*grad(xi|eta|zeta), iJ = 1/J, all rounded to FP32.  The
 // pressure E - rho u^2/2 carries rounding of E's size, so 1e-6 of E is added to
 // it; |u.A| carries rounding of |u||A|'s size, so 1e-6 (|u|+|v|+|w|) is added to
 // the sound speed; the remaining 40 roundings are covered by the factor 1 +
-// 2e-5.  small: the least |A|^2 (below 1e-30 its square root flushes to zero and
-// the bound holds nothing).
+// 2e-5.  small: the least of the |A|^2 (below 1e-30 a square root flushes to zero
+// and the bound holds nothing) and of c^2 less 2.5e-6 gamma (gamma-1) |E|/rho.
+// The padded pressure exceeds the FP64 one by at most 1.7e-6 of E ((gamma-1)
+// aside), so a node whose FP64 pressure is not positive has a negative small;
+// an ordinary node comes near that only above Mach 1000.
 template <typename R>
 __device__ __forceinline__ R sigma_bound(const R q[5], const R A[9], R iJ, float gamma, float gam1, R& small) {
   const R i = rcp_(q[0]);
   const R u = ml(q[1], i), v = ml(q[2], i), w = ml(q[3], i);
   const R k = fm(q[3], w, fm(q[2], v, ml(q[1], u)));
   const R p = ml(cst<R>(gam1), fm(cst<R>(-0.5), k, ml(cst<R>(1.0 + 1.0e-6), q[4])));
-  const R c = fm(cst<R>(1.0e-6), ad(abs_(u), ad(abs_(v), abs_(w))), sqrt_(ml(ml(cst<R>(gamma), p), i)));
+  const R c2 = ml(ml(cst<R>(gamma), p), i);
+  const R c = fm(cst<R>(1.0e-6), ad(abs_(u), ad(abs_(v), abs_(w))), sqrt_(c2));
+  small = fm(cst<R>(-2.5e-6 * gamma * gam1), abs_(ml(q[4], i)), c2);
   R s = cst<R>(0.0);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const R x = A[3 * d], y = A[3 * d + 1], z = A[3 * d + 2];
     const R nn = fm(z, z, fm(y, y, ml(x, x)));
-    small = d == 0 ? nn : neg(max_(neg(small), neg(nn)));
+    small = min_(small, nn);
     s = ad(s, fm(c, sqrt_(nn), abs_(fm(w, z, fm(v, y, ml(u, x))))));
   }
   return ml(s, ml(abs_(iJ), cst<R>(1.0 + 2.0e-5)));

@@ -237,7 +237,7 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
         const float qm = fabsf(fu) + fabsf(fv) + fabsf(fw);
         const float c = sqrt_(ft) * (float)a.Mach_inv;
         const float vis = 2.f * (float)mu * (float)a.C_dt_v * ir * (a.dt_full ? 1.f : qm * rcp_(c)) * fi;
-        float b = 0.f, small = 1.f;
+        float b = 0.f, small = ft;  // a T that flushes to zero in FP32 may be negative
 #pragma unroll
         for (int dd = 0; dd < 3; ++dd) {
           const float x = (float)m9[3 * dd], y = (float)m9[3 * dd + 1], z = (float)m9[3 * dd + 2];
