@@ -28,7 +28,7 @@
 //     (w0,w2 = A +- B, w1 = f0 - 2A, w3,w4 = tangential momenta) and the right
 //     eigenvectors likewise, instead of 5x5 matrix products; the second
 //     tangent is the cross product of the unit normal and the first;
-//   * each WENO5 value takes one reciprocal (weights scaled by the product of
+//   * an FP64 WENO5 value takes one reciprocal (weights scaled by the product of
 //     the squared indicators);
 //   * the Lax-Friedrichs flux is formed from the reconstructed conservative
 //     values, each side's collected into one coefficient ((q_n +- ws)/2).
@@ -217,9 +217,9 @@ __device__ __forceinline__ F2 half_abs(F2 x) {
   return each(x, [](float a) { return ml(0.5f, fabsf(a)); });
 }
 
-// Scale of the differences WENO5 works on: the indicators' fourth powers stay
-// inside FP32 for differences up to 7e5 (eps enters at 4e-9); FP64 takes the
-// 1/6 of the candidate values here.
+// Scale of the differences WENO5 works on: in FP32 the indicators and the squares
+// of their reciprocals stay in range for differences up to 1e10 (eps enters at
+// 4e-9); FP64 takes the 1/6 of the candidate values here.
 template <typename R>
 struct WenoScale {
   static constexpr bool d = sizeof(typename Elem<R>::T) == 8;
@@ -240,7 +240,21 @@ __device__ __forceinline__ void weno5_pair(R g1, R g2, R g3, R g4, R g5, R eps4,
   auto side = [](R e1, R e2, R e3, R t1, R t2, R t3, R gn, R gc, R* out) {
     // gn, gc: the difference next to the far pair and the one across the face
     const R s1 = fm(e1, e1, t1), s2 = fm(e2, e2, t2), s3 = fm(e3, e3, t3);
-    const R p1 = ml(s2, s3), p2 = ml(s1, s3), p3 = ml(s1, s2);
+    // the weights' square roots, up to a common factor.  FP64: one reciprocal in
+    // all.  FP32: one per indicator -- products of two indicators, squared, leave
+    // the range from differences of 2e5 on; scaling them back into it took
+    // longer (split 193x161x129, 40 steps: 66.0 ms with the bare products, 69.8
+    // scaled, 67.9 with the reciprocals).
+    R p1, p2, p3;
+    if constexpr (sizeof(typename Elem<R>::T) == 4) {
+      p1 = rcp_(s1);
+      p2 = rcp_(s2);
+      p3 = rcp_(s3);
+    } else {
+      p1 = ml(s2, s3);
+      p2 = ml(s1, s3);
+      p3 = ml(s1, s2);
+    }
     const R u1 = ml(p1, p1), u2 = ml(cst<R>(6.0), ml(p2, p2)), u3 = ml(cst<R>(3.0), ml(p3, p3));
     const R q1 = twice_less(e1, gn), q2 = ad(e2, gc), q3 = ad(e3, gc);
     const R n = fm(u3, q3, fm(u2, q2, ml(u1, q1)));
