@@ -4,6 +4,7 @@
 #include <cuda.h>
 
 #include "cbns_common.cuh"
+#include "tma.cuh"
 
 namespace cbns {
 
@@ -18,6 +19,7 @@ namespace cbns {
 struct StageMaps {
   CUtensorMap q_a, q_b, xi, eta, zeta, q0, qp, iJ, dfv;
 };
+constexpr int kStageMaps = sizeof(StageMaps) / sizeof(CUtensorMap);
 
 struct StageCore {
   Dims d;
@@ -52,6 +54,14 @@ __device__ __forceinline__ void copy_core(StageCore* to, const StageCore* from, 
   const int* src = reinterpret_cast<const int*>(from);
   int* dst = reinterpret_cast<int*>(to);
   for (int e = threadIdx.x; e < (int)(sizeof(StageCore) / sizeof(int)); e += nt) dst[e] = __ldg(src + e);
+}
+
+// The tensor maps of batch item `blk`, once per CTA and block (thread 0, which
+// alone uses them; `have`: the block of its last item, -1 at first).
+__device__ __forceinline__ void batch_maps(const StageArgs* args, int blk, int& have) {
+  if (threadIdx.x != 0 || blk == have) return;
+  have = blk;
+  tma::acquire_maps(&args[blk].tm.q_a, kStageMaps);
 }
 
 // Many blocks in one launch (a persistent work queue): args[b] are the

@@ -498,6 +498,7 @@ __global__ void __launch_bounds__(NT, 3) stage32_kernel_batched(const BatchStage
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ StageCore args;
   __shared__ int item;
+  int maps_of = -1;
   for (;;) {
     if (threadIdx.x == 0) item = (int)atomicAdd(b.counter, 1u);
     __syncthreads();
@@ -505,6 +506,7 @@ __global__ void __launch_bounds__(NT, 3) stage32_kernel_batched(const BatchStage
     if (w >= b.total) break;
     const int blk = block_of_cta(b.start, b.nblocks, w);
     copy_core(&args, b.args + blk, NT);
+    batch_maps(b.args, blk, maps_of);
     __syncthreads();
     const int local = w - __ldg(b.start + blk);
     const int ntiles = args.ntile_i * args.ntile_j;

@@ -75,6 +75,14 @@ __device__ __forceinline__ void load_4d(void* dst, const CUtensorMap* map, int x
       : "memory");
 }
 
+// Before this thread uses `n` maps that lie in global memory: a copy wrote them
+// there, and the unit that reads them keeps its own cache of them.  (A map in a
+// kernel's parameters needs none.)
+__device__ __forceinline__ void acquire_maps(const CUtensorMap* maps, int n) {
+  for (int m = 0; m < n; ++m)
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(maps + m) : "memory");
+}
+
 // the same box's lines into L2
 __device__ __forceinline__ void prefetch_4d(const CUtensorMap* map, int x, int y, int z, int f) {
   asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(
