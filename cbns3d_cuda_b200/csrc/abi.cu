@@ -34,10 +34,6 @@ namespace cbns {
 cudaError_t launch_mlp_predict_tc(const float* P, const float* X, unsigned n, float* out, int* fail, cudaStream_t s);
 }
 
-namespace cbns {
-void stage_prepare();
-}
-
 enum { PK_STAGE = 0, PK_BC = 1, PK_VISC = 2, PK_STEP = 3, PK_SENSOR = 4, PK_AUDIT = 5, PK_WENO = 6, PK_N = 7 };
 
 struct cbns_ctx {
@@ -1184,8 +1180,12 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   c->kchunk = fp32 ? kchunk_by_waves(ntiles, nint, slots, 0.5) : kchunk_for_waves(ntiles, nint, slots, 9.0);
   if ((long)ntiles * ((nint + c->kchunk - 1) / c->kchunk) < 4L * slots)
     c->kchunk = kchunk_small(d, ntiles, c->nsm, per_sm);
-  if (fp32) stage32_prepare();
-  else stage_prepare();
+  if (const cudaError_t e = fp32 ? stage32_prepare() : stage_prepare(); e != cudaSuccess) {
+    cudaGetLastError();
+    g_last = std::string("stage kernel attributes: ") + cudaGetErrorString(e);
+    cbns_destroy(c);
+    return CBNS_ERR_CUDA;
+  }
   if (p->precision == CBNS_PREC_HYBRID) (void)weno_prepare();
   if (cudaStreamSynchronize(c->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     g_last = "context initialisation failed";

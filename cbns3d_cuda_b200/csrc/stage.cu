@@ -28,6 +28,8 @@
 // FP32-flux precisions run stage32.cu.
 // HBM traffic per node and stage: the stage input (40 B, halos from L2), area
 // vectors and 1/J (80 B), the RK base (0-40 B) and the output (40 B).
+#include <mutex>
+
 #include "cbns_common.cuh"
 #include "face_flux.cuh"
 #include "sigma.cuh"
@@ -593,16 +595,10 @@ cudaError_t launch_t(const StageArgs& a, cudaStream_t s) {
 }
 
 template <bool VISC, bool TMA>
-void prepare_v() {
-  // the largest shared-memory carveout, so that 2 CTAs fit on an SM
-  auto set = [](const void* f) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem<TMA>());
-    cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  };
-  set((const void*)stage_kernel<VISC, 0, TMA>);
-  set((const void*)stage_kernel<VISC, 1, TMA>);
-  set((const void*)stage_kernel<VISC, 2, TMA>);
-  set((const void*)stage_kernel<VISC, 3, TMA>);
+cudaError_t prepare_v() {
+  const void* f[] = {(const void*)stage_kernel<VISC, 0, TMA>, (const void*)stage_kernel<VISC, 1, TMA>,
+                     (const void*)stage_kernel<VISC, 2, TMA>, (const void*)stage_kernel<VISC, 3, TMA>};
+  return raise_smem(f, 4, stage_smem<TMA>());
 }
 
 template <bool VISC, bool TMA>
@@ -617,16 +613,28 @@ cudaError_t launch_v(const StageArgs& a, int mode, cudaStream_t s) {
 
 }  // namespace
 
-// Raise the dynamic shared-memory limit of every instantiation once (outside
-// any stream capture).
-void stage_prepare() {
+cudaError_t raise_smem(const void* const* kernels, int n, size_t bytes) {
+  cudaError_t e = cudaSuccess;
+  for (int m = 0; m < n && e == cudaSuccess; ++m) {
+    e = cudaFuncSetAttribute(kernels[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    // the largest carveout, so that as many CTAs as the kernel is built for fit on an SM
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernels[m], cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  }
+  return e;
+}
+
+cudaError_t stage_prepare() {
+  static std::mutex m;
   static bool done = false;
-  if (done) return;
-  prepare_v<false, false>();
-  prepare_v<false, true>();
-  prepare_v<true, false>();
-  prepare_v<true, true>();
-  done = true;
+  std::lock_guard<std::mutex> lock(m);
+  if (done) return cudaSuccess;
+  cudaError_t e = prepare_v<false, false>();
+  if (e == cudaSuccess) e = prepare_v<false, true>();
+  if (e == cudaSuccess) e = prepare_v<true, false>();
+  if (e == cudaSuccess) e = prepare_v<true, true>();
+  done = e == cudaSuccess;
+  return e;
 }
 
 void stage_tiles(const Dims& d, int* ntile_i, int* ntile_j) {

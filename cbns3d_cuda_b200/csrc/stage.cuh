@@ -79,8 +79,13 @@ struct BatchStage {
 // variant: a compiled occupancy variant, 0 .. stage_variants(fp32)-1.
 cudaError_t launch_stage(const StageArgs& a, int mode, bool visc, bool fp32, int variant, cudaStream_t s);
 int stage_variants(bool fp32, bool hybrid);
+// Raise the dynamic shared-memory limits of every stage kernel of the precision,
+// once per process, outside any stream capture: returns when they are raised,
+// whichever thread does it, and is tried again after a failure.
+cudaError_t stage_prepare();
+cudaError_t stage32_prepare();
+cudaError_t raise_smem(const void* const* kernels, int n, size_t bytes);
 // The FP32 kernels (stage32.cu); variant 0: registers for 2 CTAs per SM, else 3.
-void stage32_prepare();
 cudaError_t launch_stage32(const StageArgs& a, int mode, bool visc, int variant, cudaStream_t s);
 cudaError_t launch_stage32_batched(const BatchStage& b, int mode, bool visc, bool hybrid, cudaStream_t s);
 // Hybrid: evaluate the listed faces (the widening pass's lists; every face

@@ -44,6 +44,8 @@
 // kernel by the WENO5-face pass (weno_faces.cu) and read from its face array.
 // The decisions of plane k+1 are read while plane k is computed, and the WENO5
 // fluxes of plane k are asked into L1 at its start.
+#include <mutex>
+
 #include "cbns_common.cuh"
 #include "face_flux.cuh"
 #include "sigma.cuh"
@@ -569,33 +571,32 @@ cudaError_t launch_h(const StageArgs& a, int mode, bool visc, cudaStream_t s) {
 }
 
 template <bool VISC, bool HYB, int NB>
-void prepare_v() {
-  auto set = [](const void* f) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
-    cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  };
-  set((const void*)stage32_kernel<VISC, 0, HYB, NB>);
-  set((const void*)stage32_kernel<VISC, 1, HYB, NB>);
-  set((const void*)stage32_kernel<VISC, 2, HYB, NB>);
-  set((const void*)stage32_kernel<VISC, 3, HYB, NB>);
+cudaError_t prepare_v() {
+  const void* f[] = {(const void*)stage32_kernel<VISC, 0, HYB, NB>, (const void*)stage32_kernel<VISC, 1, HYB, NB>,
+                     (const void*)stage32_kernel<VISC, 2, HYB, NB>, (const void*)stage32_kernel<VISC, 3, HYB, NB>};
+  return raise_smem(f, 4, kSmem);
 }
 
 template <int NB>
-void prepare_nb() {
-  prepare_v<false, false, NB>();
-  prepare_v<false, true, NB>();
-  prepare_v<true, false, NB>();
-  prepare_v<true, true, NB>();
+cudaError_t prepare_nb() {
+  cudaError_t e = prepare_v<false, false, NB>();
+  if (e == cudaSuccess) e = prepare_v<false, true, NB>();
+  if (e == cudaSuccess) e = prepare_v<true, false, NB>();
+  if (e == cudaSuccess) e = prepare_v<true, true, NB>();
+  return e;
 }
 
 }  // namespace
 
-void stage32_prepare() {
+cudaError_t stage32_prepare() {
+  static std::mutex m;
   static bool done = false;
-  if (done) return;
-  done = true;
-  prepare_nb<2>();
-  prepare_nb<3>();
+  std::lock_guard<std::mutex> lock(m);
+  if (done) return cudaSuccess;
+  cudaError_t e = prepare_nb<2>();
+  if (e == cudaSuccess) e = prepare_nb<3>();
+  done = e == cudaSuccess;
+  return e;
 }
 
 cudaError_t launch_stage32(const StageArgs& a, int mode, bool visc, int variant, cudaStream_t s) {
