@@ -54,7 +54,7 @@ def _run(cmd: list[str]) -> None:
 def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(parents=True, exist_ok=True)
     (PKG / "bin").mkdir(exist_ok=True)
-    headers = list(CSRC.glob("*.cuh")) + list((ROOT / "include").glob("*.h"))
+    headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list((ROOT / "include").glob("*.h"))
     srcs = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp"))
     nvcc = _nvcc()
     jobs = []

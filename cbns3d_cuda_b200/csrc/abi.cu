@@ -23,6 +23,7 @@
 #include "cbns_common.cuh"
 #include "setup.cuh"
 #include "stage.cuh"
+#include "kchunk.h"
 #include "step.cuh"
 #include "tma.cuh"
 #include "visc.cuh"
@@ -122,78 +123,6 @@ int dalloc(cbns_ctx* c, double** p, size_t elems) {
 
 inline long round_up(long x, long m) { return (x + m - 1) / m * m; }
 
-// k planes per CTA of the stage kernel.  The CTAs (tiles x k chunks) run in
-// waves of `slots` (SMs x CTAs per SM); a chunk costs its planes plus some
-// warm-up (the ring's first planes and the first k-face), `warm` planes'
-// worth.  The chunk count whose waves x (planes + warm) is least, keeping
-// chunks of at least 8 planes.
-int kchunk_by_waves(int ntiles, int nint, int slots, double warm) {
-  const int maxchunk = std::max(1, nint / 8);
-  double best = 1e300;
-  int best_k = nint;
-  for (int nchunk = 1; nchunk <= maxchunk; ++nchunk) {
-    const int kc = (nint + nchunk - 1) / nchunk;
-    const long items = (long)ntiles * ((nint + kc - 1) / kc);
-    const long waves = (items + slots - 1) / slots;
-    const double cost = (double)waves * (kc + warm);
-    if (cost < best - 1e-9) {
-      best = cost;
-      best_k = kc;
-    }
-  }
-  return best_k;
-}
-
-// The chunk for about `waves` waves of `slots` CTAs, chunks of at least 8 planes.
-// Many short waves balance CTAs of unequal cost (tiles cut by the grid's edge,
-// WENO5 faces gathered unevenly): on a 256 x 256 x 128 grid the FP64 kernel
-// runs fastest at about 9 waves (13-plane chunks), 3.5% faster than at 4.6
-// waves (26-plane chunks) and 10% faster than in one wave.
-int kchunk_for_waves(int ntiles, int nint, int slots, double waves) {
-  const int want = (int)std::ceil(waves * slots / ntiles);
-  const int nchunk = std::max(1, std::min(want, nint / 8));
-  return (nint + nchunk - 1) / nchunk;
-}
-
-// The default: about four CTAs per slot of 2 CTAs per SM, chunks of at least 8 planes.
-int kchunk_default(int ntiles, int nint, int nsm) {
-  const int nchunk = std::max(1, std::min((4 * 2 * nsm + ntiles - 1) / ntiles, nint / 8));
-  return (nint + nchunk - 1) / nchunk;
-}
-
-// The chunk for a grid whose tiles at 8 planes a chunk or more make few waves of
-// CTAs: the least estimate of a launch's time in planes.  A chunk takes its
-// planes plus 0.7 for its start (the ring's first planes and the k-face below
-// it); while the CTAs fit the slots the launch is one chunk, beyond that the
-// work over the slots plus half a chunk of tail; CTAs alone on an SM run about
-// 1.5 times as fast as two.  Tiles cut by the grid's edge count by their
-// columns.  Measured us per step with this chunk against one of at least 8
-// planes: FP64 64x32x16 78 against 381 (8 CTAs marched the whole block while
-// 140 SMs idled), 97x61x45 245 against 272, 128x64x64 468 against 522; split
-// 64x32x16 69 against 258, 97x61x45 153 against 188; hybrid (3 per SM)
-// 64x32x16 146 against 277, 129x113x97 675 against 709.  Above about four
-// waves the chunks stay longer: at 193x161x129 4-plane chunks take 2770 us in
-// FP64 and 1618 split against 2682 and 1540 at 9.
-int kchunk_small(const Dims& d, int ntiles, int nsm, int per_sm) {
-  const int nint = d.KM - 2;
-  const double tiles = (d.IM - 2) * (d.JM - 2) / (double)(STAGE_TI * STAGE_TJ);
-  const double slots = (double)nsm * per_sm;
-  double best = 1e300;
-  int best_k = nint;
-  for (int kc = 1; kc <= nint; ++kc) {
-    const int nchunk = (nint + kc - 1) / kc;
-    const double items = (double)ntiles * nchunk, chunk = kc + 0.7;
-    const double cost = items <= nsm     ? chunk / 1.5
-                        : items <= slots ? chunk
-                                         : (std::max(1.0, tiles * nchunk / slots) + 0.5) * chunk;
-    if (cost < best - 1e-9) {
-      best = cost;
-      best_k = kc;
-    }
-  }
-  return best_k;
-}
-
 // Candidate chunkings for cbns_autotune at `per_sm` CTAs per SM (distinct values).
 std::vector<int> kchunk_candidates(const cbns_ctx* c, int per_sm) {
   const int ntiles = c->ntile_i * c->ntile_j, nint = c->d.KM - 2, slots = c->nsm * per_sm;
@@ -203,7 +132,7 @@ std::vector<int> kchunk_candidates(const cbns_ctx* c, int per_sm) {
   };
   for (double warm : {0.5, 2.0}) add(kchunk_by_waves(ntiles, nint, slots, warm));
   for (double waves : {4.0, 6.0, 9.0, 12.0}) add(kchunk_for_waves(ntiles, nint, slots, waves));
-  add(kchunk_small(c->d, ntiles, c->nsm, per_sm));
+  add(kchunk_small(c->d.IM, c->d.JM, c->d.KM, ntiles, c->nsm, per_sm));
   return v;
 }
 
@@ -1163,23 +1092,16 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
 
   stage_tiles(d, &c->ntile_i, &c->ntile_j);
   const int ntiles = c->ntile_i * c->ntile_j;
-  const int nint = d.KM - 2;
   {
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
   }
-  // until cbns_autotune says otherwise, the variants and chunks it picks on
-  // B200 for grids of a few million nodes: FP64 stages by TMA (about 10%
-  // faster than the synchronous variant) with about 9 waves of CTAs, the FP32
-  // kernels run 3 CTAs per SM (8% faster than 2) with chunks sized by the wave
-  // count and warm-up.  Where that makes fewer than four waves, the chunk of
-  // kchunk_small.
-  const int per_sm = fp32 ? 3 : 2, slots = c->nsm * per_sm;
+  // until cbns_autotune says otherwise, the variant it picks on B200 for grids of
+  // a few million nodes: FP64 stages by TMA (about 10% faster than the
+  // synchronous variant), the FP32 kernels run 3 CTAs per SM (8% faster than 2)
   c->stage_variant = 1;
-  c->kchunk = fp32 ? kchunk_by_waves(ntiles, nint, slots, 0.5) : kchunk_for_waves(ntiles, nint, slots, 9.0);
-  if ((long)ntiles * ((nint + c->kchunk - 1) / c->kchunk) < 4L * slots)
-    c->kchunk = kchunk_small(d, ntiles, c->nsm, per_sm);
+  c->kchunk = kchunk_start(d.IM, d.JM, d.KM, ntiles, c->nsm, fp32);
   if (const cudaError_t e = fp32 ? stage32_prepare() : stage_prepare(); e != cudaSuccess) {
     cudaGetLastError();
     g_last = std::string("stage kernel attributes: ") + cudaGetErrorString(e);

@@ -4,6 +4,7 @@
 #include <cuda.h>
 
 #include "cbns_common.cuh"
+#include "kchunk.h"
 #include "tma.cuh"
 
 namespace cbns {
@@ -96,7 +97,7 @@ cudaError_t launch_weno_faces(const StageArgs& a, int mode, long nfaces, const i
 cudaError_t weno_prepare();
 // modes 1..3 only; hybrid: the StageArgs carry decision masks.
 cudaError_t launch_stage_batched(const BatchStage& b, int mode, bool visc, bool fp32, bool hybrid, cudaStream_t s);
-constexpr int STAGE_TI = 16, STAGE_TJ = 15;  // columns of a CTA's tile
+constexpr int STAGE_TI = kTileI, STAGE_TJ = kTileJ;  // columns of a CTA's tile
 void stage_tiles(const Dims& d, int* ntile_i, int* ntile_j);
 
 }  // namespace cbns
