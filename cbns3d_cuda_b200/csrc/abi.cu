@@ -219,6 +219,7 @@ ViscArgs visc_args(cbns_ctx* c, bool check_done, bool sigma) {
   for (int m = 0; m < 6; ++m) a.prim[m] = c->f.prim[m];
   for (int m = 0; m < 10; ++m) a.area[m] = c->f.area[m];
   for (int m = 0; m < 9; ++m) a.area32[m] = c->f.area32[m];
+  for (int m = 0; m < 9; ++m) a.met[m] = c->f.met[m];
   a.Mach_inv = 1.0 / c->prm.Mach;
   for (int m = 0; m < 12; ++m) a.vflux[m] = c->f.vflux[m];
   for (int m = 0; m < 4; ++m) a.dfv[m] = c->f.dfv[m];

@@ -60,23 +60,24 @@ __device__ __forceinline__ bool sigma_reaches(float b, float small, float found)
   return !(b < found) || !(small > 1.0e-30f);
 }
 
-// The spectral radius in FP64 (explicit roundings: every kernel gives the same).
+// The spectral radius in FP64, correctly rounded divisions and roots and explicit
+// roundings: every kernel gives the same.
 __device__ __forceinline__ double sigma_exact(const double q[5], const double A[9], double iJ, double gamma,
                                               double gam1) {
-  const double r = q[0], ir = rcp_(r);
+  const double r = q[0], ir = __drcp_rn(r);
   const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
   const double k = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
   const double pp = __dmul_rn(gam1, __fma_rn(-__dmul_rn(0.5, r), k, q[4]));
-  const double cs = sqrt_(__dmul_rn(__dmul_rn(gamma, pp), ir));
+  const double cs = __dsqrt_rn(__ddiv_rn(__dmul_rn(gamma, pp), r));
   double s = 0.0;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double x = A[3 * d], y = A[3 * d + 1], z = A[3 * d + 2];
+  for (int d = 0; d < 3; ++d) {  // grad(xi|eta|zeta) = A / J
+    const double x = __dmul_rn(A[3 * d], iJ), y = __dmul_rn(A[3 * d + 1], iJ), z = __dmul_rn(A[3 * d + 2], iJ);
     const double un = __fma_rn(ww, z, __fma_rn(vv, y, __dmul_rn(uu, x)));
     const double nn = __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
-    s = __dadd_rn(s, __fma_rn(cs, sqrt_(nn), fabs(un)));
+    s = __dadd_rn(s, __dadd_rn(fabs(un), __dmul_rn(cs, __dsqrt_rn(nn))));
   }
-  return __dmul_rn(s, fabs(iJ));  // left-handed grids have J < 0
+  return s;
 }
 
 // The largest spectral radius a CTA (or an earlier one) has met, as an FP32

@@ -458,7 +458,7 @@ __device__ __forceinline__ void stage_body(const StageCore& a, const StageMaps* 
 #pragma unroll
         for (int n = 0; n < NEQ; ++n) a.out[n * VOL + o] = q[n];
         if (VISC) {
-          const double r = q[0], ir = rcp_(r);
+          const double r = q[0], ir = __drcp_rn(r);
           const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
           const double ke = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
           const double pp = __dmul_rn(a.gam1, __fma_rn(-__dmul_rn(0.5, r), ke, q[4]));
@@ -467,7 +467,7 @@ __device__ __forceinline__ void stage_body(const StageCore& a, const StageMaps* 
           a.prim[2][o] = vv;
           a.prim[3][o] = ww;
           if (!a.lean) a.prim[4][o] = pp;
-          a.prim[5][o] = ml(ml(a.gM2, pp), ir);
+          a.prim[5][o] = __ddiv_rn(ml(a.gM2, pp), r);
         } else if (kSigma && a.sigma) {
           // in FP64 only where the FP32 bound reaches the largest met so far
           float qf[NEQ], small;

@@ -415,7 +415,7 @@ __device__ __forceinline__ void stage32_body(const StageCore& a, const StageMaps
           a.out32[n * VOL + o] = qf[q2][n] = (float)q[n];
         }
         if (VISC) {
-          const double r = q[0], ir = rcp_(r);
+          const double r = q[0], ir = __drcp_rn(r);
           const double uu = __dmul_rn(q[1], ir), vv = __dmul_rn(q[2], ir), ww = __dmul_rn(q[3], ir);
           const double kk = __fma_rn(ww, ww, __fma_rn(vv, vv, __dmul_rn(uu, uu)));
           const double pp = __dmul_rn(a.gam1, __fma_rn(-__dmul_rn(0.5, r), kk, q[4]));
@@ -424,7 +424,7 @@ __device__ __forceinline__ void stage32_body(const StageCore& a, const StageMaps
           a.prim[2][o] = vv;
           a.prim[3][o] = ww;
           if (!a.lean) a.prim[4][o] = pp;
-          a.prim[5][o] = ml(ml(a.gM2, pp), ir);
+          a.prim[5][o] = __ddiv_rn(ml(a.gM2, pp), r);
         }
       }
     }

@@ -79,6 +79,39 @@ __device__ __forceinline__ void halo_node(int h, int i0, int j0, int& gi, int& g
   }
 }
 
+// The spectral radius of the node at o in FP64, from the FP64 fields whatever the
+// kernel's arithmetic (src/time_step_kernel.cu:13-96), with correctly rounded
+// divisions and roots.
+// AHEAD: all loads in flight before the first use (met is not in cache: 128x64x64,
+// node and divergence launches of a step 238 -> 222 us); the FP32 kernels, built
+// for 64 registers, spill with it.
+template <bool AHEAD>
+__device__ __forceinline__ double sigma_node(const ViscArgs& a, long o) {
+  double m[9];  // grad(xi|eta|zeta)
+  if (AHEAD) {
+#pragma unroll
+    for (int n = 0; n < 9; ++n) m[n] = __ldg(a.met[n] + o);
+  }
+  const double r = __ldg(a.prim[0] + o), T = __ldg(a.prim[5] + o), p = __ldg(a.prim[4] + o);
+  const double u = __ldg(a.prim[1] + o), v = __ldg(a.prim[2] + o), w = __ldg(a.prim[3] + o);
+  const double mu = (1.0 + a.C_T_inf) / (T + a.C_T_inf) * sqrt(T * T * T);
+  const double c = sqrt(a.gamma * p / r);
+  const double fv = a.dt_full ? 2.0 * mu * a.C_dt_v / r : 2.0 * mu * a.C_dt_v * sqrt(u * u + v * v + w * w) / c / r;
+  auto part = [&](double x, double y, double z) {
+    const double na = sqrt(x * x + y * y + z * z);
+    return fabs(u * x + v * y + w * z) + c * na + na * na * fv;
+  };
+  double s = 0.0;
+  if (AHEAD) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s += part(m[3 * d], m[3 * d + 1], m[3 * d + 2]);
+  } else {
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) s += part(__ldg(a.met[3 * d] + o), __ldg(a.met[3 * d + 1] + o), __ldg(a.met[3 * d + 2] + o));
+  }
+  return s;
+}
+
 // CTA `cta` of one block's node-kernel grid (tiles in i, then j, then k chunks).
 // Every thread of the CTA calls this (block-wide barriers; the spectral-radius
 // maximum is a warp reduction).
@@ -155,6 +188,8 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
       load_ring(k + 3, rn);
       load_halo(k + 1, hn);
     }
+    float upper = 0.f, lower = 0.f, small = 1.f;
+    bool node = false;  // a grid node whose spectral radius counts
     if (valid) {
       const long o = o_own + k * sk;
       // the node's area vectors J*grad(xi|eta|zeta) and 1/J: the gradients'
@@ -194,7 +229,7 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
       const T uu = c4[0][VH + ty][VH + tx], vv = c4[1][VH + ty][VH + tx], ww = c4[2][VH + ty][VH + tx];
       const T Tl = c4[3][VH + ty][VH + tx];
       const T CT = (T)a.C_T_inf;
-      const T mu = ml((T(1) + CT) * Tl * sqrt_(Tl), rcp_(Tl + CT));
+      const T mu = (T(1) + CT) / (Tl + CT) * sqrt(Tl * Tl * Tl);
       if (a.keep_mu) a.mu[o] = (double)mu;
       // chain rule: d/dx = xi_x d/dxi + eta_x d/deta + zeta_x d/dzeta, etc.
       const T ux = gx[0] * m9[0] + ge[0] * m9[3] + gz[0] * m9[6];
@@ -228,45 +263,42 @@ __device__ __forceinline__ void visc_node_tile(const ViscArgs& a, int cta, ViscS
       }
       const int i = gi - NG, j = gj - NG, kk = k - NG;
       if (a.sigma && i >= 0 && i < d.IM && j >= 0 && j < d.JM && kk >= 0 && kk < d.KM) {
-        // the spectral radius for the next dt (src/time_step_kernel.cu:13-96):
-        // FP64 from the FP64 fields, where an FP32 bound of it (rounded values,
-        // c = sqrt(T)/M; the roundings covered by 1e-6 |u||A| and 2e-5) reaches
-        // the largest met so far
+        // FP32 bounds of the node's spectral radius: rounded values, c = sqrt(T)/M;
+        // the roundings covered by 1e-6 |u||A| and 2e-5.  The viscous part, with
+        // |u|+|v|+|w| for |u|, in the upper one only
         const float fu = (float)uu, fv = (float)vv, fw = (float)ww, ft = (float)Tl, fi = fabsf((float)iJ);
         const float ir = rcp_((float)__ldg(a.prim[0] + o));
         const float qm = fabsf(fu) + fabsf(fv) + fabsf(fw);
         const float c = sqrt_(ft) * (float)a.Mach_inv;
         const float vis = 2.f * (float)mu * (float)a.C_dt_v * ir * (a.dt_full ? 1.f : qm * rcp_(c)) * fi;
-        float b = 0.f, small = ft;  // a T that flushes to zero in FP32 may be negative
+        float b = 0.f, e = 0.f, g = 0.f;
+        small = ft;  // a T that flushes to zero in FP32 may be negative
 #pragma unroll
         for (int dd = 0; dd < 3; ++dd) {
           const float x = (float)m9[3 * dd], y = (float)m9[3 * dd + 1], z = (float)m9[3 * dd + 2];
-          const float nn = fm(z, z, fm(y, y, ml(x, x)));
+          const float nn = fm(z, z, fm(y, y, ml(x, x))), n1 = sqrt_(nn);
           small = fminf(small, nn);
-          b += fabsf(fm(fw, z, fm(fv, y, ml(fu, x)))) + fm(1.0e-6f, qm, c) * sqrt_(nn) + nn * vis;
+          b += fabsf(fm(fw, z, fm(fv, y, ml(fu, x)))) + c * n1;
+          e += n1;
+          g += nn;
         }
-        b *= fi * (1.f + 2.0e-5f);
-        if (sigma_reaches(b, small, __int_as_float(*(volatile int*)&sm.best))) {
-          const double ud = __ldg(a.prim[1] + o), vd = __ldg(a.prim[2] + o), wd = __ldg(a.prim[3] + o);
-          const double Td = __ldg(a.prim[5] + o), ird = rcp_(__ldg(a.prim[0] + o));
-          const double J1 = fabs(__ldg(a.area[9] + o));
-          const double cd = sqrt_(a.gamma * __ldg(a.prim[4] + o) * ird);
-          const double mud = (1.0 + a.C_T_inf) * Td * sqrt_(Td) * rcp_(Td + a.C_T_inf);
-          const double fvd = 2.0 * mud * a.C_dt_v * ird * (a.dt_full ? 1.0 : sqrt_(ud * ud + vd * vd + wd * wd) * rcp_(cd));
-          double s = 0.0;
-#pragma unroll 1
-          for (int dd = 0; dd < 3; ++dd) {
-            const double mx = __ldg(a.area[3 * dd] + o), my = __ldg(a.area[3 * dd + 1] + o),
-                         mz = __ldg(a.area[3 * dd + 2] + o);
-            const double nn = mx * mx + my * my + mz * mz;
-            s += fabs(ud * mx + vd * my + wd * mz) + cd * sqrt_(nn) + nn * J1 * fvd;
-          }
-          s *= J1;
-          if (s != s) nanseen = true;
-          else if (!has || s > sg) sg = s;
-          has = true;
-          sigma_found(&sm.best, s);
-        }
+        e *= 1.0e-6f * qm;
+        upper = (b + e + g * vis) * (fi * (1.f + 2.0e-5f));
+        lower = (b - e) * (fi * (1.f - 2.0e-5f));
+        node = true;
+      }
+    }
+    if (a.sigma) {
+      // the spectral radius for the next dt, in FP64 where the upper bound reaches
+      // the largest met so far or known to be in the warp
+      const bool use = lower > 0.f && lower < 1.0e38f;
+      const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, use ? __float_as_uint(lower) : 0u));
+      if (node && sigma_reaches(upper, small, fmaxf(most, __int_as_float(*(volatile int*)&sm.best)))) {
+        const double s = sigma_node<sizeof(T) == 8>(a, o_own + k * sk);
+        if (s != s) nanseen = true;
+        else if (!has || s > sg) sg = s;
+        has = true;
+        sigma_found(&sm.best, s);
       }
     }
     // the ring is the thread's own column, plane k+1's buffer was last read

@@ -13,6 +13,7 @@ struct ViscArgs {
   const double* prim[6];     // rho,u,v,w,p,T
   const double* area[10];    // J*grad(xi|eta|zeta), 1/J
   const float* area32[9];    // their FP32 copies (f32)
+  const double* met[9];      // grad(xi|eta|zeta): the FP64 spectral radius
   double Mach_inv;
   double* vflux[12];         // E0..E3, F0..F3, G0..G3 (FP32 elements when f32)
   double* dfv[4];            // their divergence at the interior nodes (FP32 elements when f32)
