@@ -47,7 +47,6 @@ struct cbns_ctx {
   int lq = 0, lp = 1, ls = 2;  // physical index of logical Q, Q_p, spare
   Fields f;
   double* staging = nullptr;
-  size_t staging_elems = 0;
   StepState* st = nullptr;
   unsigned* counter = nullptr;  // device counter for face sampling
   bool have_metrics = false, sigma_valid = false;
@@ -393,7 +392,7 @@ SensorSet sensor_set(cbns_ctx* c, const double* q, bool check_done, bool every_s
   a.gam1 = (float)c->ph.gam1;
   a.gam1_inv = (float)c->ph.gam1_inv;
   a.q = copy32(c, q);
-  for (int k = 0; k < 10; ++k) a.area[k] = c->f.area[k];
+  fill_met(c, a.met);
   a.mask = c->mask;
   a.stride = c->audit_stride;
   a.bound = c->audit_bound;
@@ -971,15 +970,18 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   int rc = CBNS_OK;
   for (int b = 0; b < 3 && rc == CBNS_OK; ++b) rc = dalloc(c, &c->qb[b], (size_t)NEQ * d.VOL);
   for (int m = 0; m < 10 && rc == CBNS_OK; ++m) rc = dalloc(c, &c->f.met[m], d.VOL);
+  const bool fp32 = p->precision != CBNS_PREC_FP64;
   {
-    // one allocation, components VOL elements apart (one 4-D tensor map covers them)
+    // one allocation, components VOL elements apart (one 4-D tensor map covers
+    // them); with the FP32 flux J*grad(zeta) and 1/J only
+    const int m0 = fp32 ? 6 : 0;
     double* tmp = nullptr;
-    rc = rc == CBNS_OK ? dalloc(c, &tmp, (size_t)10 * d.VOL) : rc;
+    for (int m = 0; m < 10; ++m) c->f.area[m] = nullptr;
+    rc = rc == CBNS_OK ? dalloc(c, &tmp, (size_t)(10 - m0) * d.VOL) : rc;
     if (rc == CBNS_OK)
-      for (int m = 0; m < 10; ++m) c->f.area[m] = tmp + (size_t)m * d.VOL;
+      for (int m = m0; m < 10; ++m) c->f.area[m] = tmp + (size_t)(m - m0) * d.VOL;
   }
   for (int m = 0; m < 9; ++m) c->f.area32[m] = nullptr;
-  const bool fp32 = p->precision != CBNS_PREC_FP64;
   if (fp32) {
     // one allocation, components VOL floats apart (one 4-D tensor map covers
     // them); the same for each state buffer's FP32 copy
@@ -992,7 +994,8 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
       c->q32[b] = reinterpret_cast<float*>(tmp);
     }
   }
-  for (int m = 0; m < 7 && rc == CBNS_OK; ++m) rc = dalloc(c, &c->f.prim[m], d.VOL);
+  for (int m = 0; m < 7; ++m) c->f.prim[m] = nullptr;
+  for (int m = 0; m < (p->viscous ? 7 : 6) && rc == CBNS_OK; ++m) rc = dalloc(c, &c->f.prim[m], d.VOL);
   for (int m = 0; m < 12; ++m) c->f.vflux[m] = nullptr;
   for (int m = 0; m < 4; ++m) c->f.dfv[m] = nullptr;
   if (p->viscous) {
@@ -1002,9 +1005,8 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
     rc = rc == CBNS_OK ? dalloc(c, &tmp, (size_t)4 * d.VOL) : rc;
     for (int m = 0; m < 4 && rc == CBNS_OK; ++m) c->f.dfv[m] = tmp + (size_t)m * d.VOL;
   }
-  const long NGt = (long)d.IG * d.JG * d.KG;
-  c->staging_elems = (size_t)std::max(5 * NGt, 10L * d.IM * d.JM * d.KM);
-  if (rc == CBNS_OK) rc = dalloc(c, &c->staging, c->staging_elems);
+  // a whole state, the largest array that goes through it
+  if (rc == CBNS_OK) rc = dalloc(c, &c->staging, (size_t)NEQ * d.IG * d.JG * d.KG);
   c->nfaces = (long)(d.IM - 1) * (d.JM - 2) * (d.KM - 2) + (long)(d.IM - 2) * (d.JM - 1) * (d.KM - 2) +
               (long)(d.IM - 2) * (d.JM - 2) * (d.KM - 1);
   if (rc == CBNS_OK && p->precision == CBNS_PREC_HYBRID && (c->nfaces >= (1L << 31) || d.VOL >= (1L << 30))) {
@@ -1064,7 +1066,7 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
       ok = ok && encode_node_map(&m.eta, ar, es, d.PX, d.JG, d.KG, d.VOL, na, 16, 17, 3);
       ok = ok && encode_node_map(&m.zeta, ar, es, d.PX, d.JG, d.KG, d.VOL, na, 16, 15, 3);
       ok = ok && encode_node_map(&c->tm_rk[b], c->qb[b], 8, d.PX, d.JG, d.KG, d.VOL, NEQ, 16, 15, NEQ);
-      ok = ok && encode_node_map(&m.iJ, c->f.area[0], 8, d.PX, d.JG, d.KG, d.VOL, 10, 16, 15, 1);
+      ok = ok && encode_node_map(&m.iJ, c->f.area[9], 8, d.PX, d.JG, d.KG, d.VOL, 1, 16, 15, 1);
       m.q0 = m.qp = c->tm_rk[b];
       m.dfv = m.iJ;  // FP32 kernels of viscous runs only
       if (p->viscous && fp32)  // FP32 elements in arrays VOL doubles apart
@@ -1080,12 +1082,14 @@ int cbns_create(const cbns_params* p, cbns_ctx** out) {
   for (void* a : c->allocs) (void)a;
   for (int b = 0; b < 3; ++b) cudaMemsetAsync(c->qb[b], 0, (size_t)NEQ * d.VOL * sizeof(double), c->stream);
   for (int m = 0; m < 10; ++m) cudaMemsetAsync(c->f.met[m], 0, d.VOL * sizeof(double), c->stream);
-  for (int m = 0; m < 10; ++m) cudaMemsetAsync(c->f.area[m], 0, d.VOL * sizeof(double), c->stream);
+  for (int m = 0; m < 10; ++m)
+    if (c->f.area[m]) cudaMemsetAsync(c->f.area[m], 0, d.VOL * sizeof(double), c->stream);
   for (int m = 0; m < 9; ++m)
     if (c->f.area32[m]) cudaMemsetAsync(c->f.area32[m], 0, d.VOL * sizeof(float), c->stream);
   for (int b = 0; b < 3; ++b)
     if (c->q32[b]) cudaMemsetAsync(c->q32[b], 0, (size_t)NEQ * d.VOL * sizeof(float), c->stream);
-  for (int m = 0; m < 7; ++m) cudaMemsetAsync(c->f.prim[m], 0, d.VOL * sizeof(double), c->stream);
+  for (int m = 0; m < 7; ++m)
+    if (c->f.prim[m]) cudaMemsetAsync(c->f.prim[m], 0, d.VOL * sizeof(double), c->stream);
   if (p->viscous) {
     for (int m = 0; m < 12; ++m) cudaMemsetAsync(c->f.vflux[m], 0, d.VOL * sizeof(double), c->stream);
     for (int m = 0; m < 4; ++m) cudaMemsetAsync(c->f.dfv[m], 0, d.VOL * sizeof(double), c->stream);
@@ -1456,7 +1460,7 @@ int cbns_sensor_sample(cbns_ctx* c, int which, unsigned stride, unsigned offset,
   a.gamma = (float)c->ph.gamma;
   a.gam1 = (float)c->ph.gam1;
   a.q = buf(c, which);
-  for (int m = 0; m < 10; ++m) a.area[m] = c->f.area[m];
+  fill_met(c, a.met);
   a.stride = stride;
   a.offset = offset;
   a.feat = feat;

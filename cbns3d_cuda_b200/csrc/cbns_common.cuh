@@ -34,6 +34,11 @@ __host__ __device__ inline long node_off(const Dims& d, int i, int j, int k) {
   return LP + (long)(i + NG) + d.PX * ((long)(j + NG) + (long)d.JG * (long)(k + NG));
 }
 
+// Component m of a node's area vectors: J grad(xi) (0..2), J grad(eta), J grad(zeta).
+__device__ __forceinline__ double node_area(const double* const met[10], int m, long o) {
+  return __dmul_rn(met[m][o], met[9][o]);
+}
+
 // Physical parameters after the derivation of src/Block3d.cpp:99-113.
 struct Phys {
   double gamma, gam1, gam1_inv, gM2, Mach2, p_inf, CFL, Re_inv, Pr_inv, C_T_inf, C_dt_v;
@@ -45,9 +50,9 @@ struct Phys {
 // Device pointers of one context.  Q buffers hold 5 fields each.
 struct Fields {
   double* met[10];   // xi_x, xi_y, xi_z, eta_x, eta_y, eta_z, zeta_x, zeta_y, zeta_z, Jac
-  double* area[10];  // J*grad(xi) (3), J*grad(eta) (3), J*grad(zeta) (3), 1/J
+  double* area[10];  // J*grad(xi) (3), J*grad(eta) (3), J*grad(zeta) (3), 1/J; FP32-flux contexts: the last four
   float* area32[9];  // FP32-flux contexts: J*grad(xi), J*grad(eta), J*grad(zeta) rounded to FP32
-  double* prim[7];   // rho, u, v, w, p, T, mu (viscous upkeep; on-demand otherwise)
+  double* prim[7];   // rho, u, v, w, p, T, mu (viscous upkeep; on-demand and without mu otherwise)
   double* vflux[12]; // E0..E3, F0..F3, G0..G3 (viscous node fluxes, times J-scaled normals)
   double* dfv[4];    // divergence of the viscous node fluxes at the interior nodes (momentum 3, energy)
 };

@@ -44,8 +44,12 @@ __global__ void sample_faces_kernel(const SampleArgs a) {
   auto ld = [&](int p, int n) -> float { return (float)q[n * V + oa + (p - 2) * sd]; };
   // the same FP32 arithmetic as the per-step sensor sweep, so that inference
   // sees exactly the features the network was trained on
-  const float A[3] = {(float)a.area[3 * dir][oa], (float)a.area[3 * dir + 1][oa], (float)a.area[3 * dir + 2][oa]};
-  const float B[3] = {(float)a.area[3 * dir][ob], (float)a.area[3 * dir + 1][ob], (float)a.area[3 * dir + 2][ob]};
+  float A[3], B[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    A[m] = (float)node_area(a.met, 3 * dir + m, oa);
+    B[m] = (float)node_area(a.met, 3 * dir + m, ob);
+  }
   float ux, uy, uz;
   face_unit_normal(A, B, ux, uy, uz);
   float f[SN_IN];
@@ -440,9 +444,8 @@ __device__ __forceinline__ void audit_body(const AuditArgs& a, unsigned bx) {
     const long sd = dir == 0 ? 1 : (dir == 1 ? d.PX : d.PL);
     const long oa = node_off(d, i, j, k), ob = oa + sd;
     auto ld = [&](int p, int n) -> float { return __ldg(a.q + n * d.VOL + oa + (p - 2) * sd); };
-    const float nx = (float)(0.5 * (__ldg(a.area[3 * dir] + oa) + __ldg(a.area[3 * dir] + ob)));
-    const float ny = (float)(0.5 * (__ldg(a.area[3 * dir + 1] + oa) + __ldg(a.area[3 * dir + 1] + ob)));
-    const float nz = (float)(0.5 * (__ldg(a.area[3 * dir + 2] + oa) + __ldg(a.area[3 * dir + 2] + ob)));
+    auto normal = [&](int m) { return (float)(0.5 * (node_area(a.met, m, oa) + node_area(a.met, m, ob))); };
+    const float nx = normal(3 * dir), ny = normal(3 * dir + 1), nz = normal(3 * dir + 2);
     const FluxConsts<float> C{a.gamma, a.gam1, a.gam1_inv};
     float fw[5], fl[5];
     face_flux<float>(ld, nx, ny, nz, C, fw);

@@ -10,7 +10,7 @@ struct SampleArgs {
   Dims d;
   float gamma, gam1;
   const double* q;          // state buffer (5 fields)
-  const double* area[10];   // node area vectors
+  const double* met[10];    // metrics and Jacobian: node area vectors are their products
   unsigned stride, offset;  // faces with (global face index % stride) == offset
   float* feat;              // capacity x 15
   unsigned char* label;     // capacity
@@ -107,7 +107,7 @@ struct AuditArgs {
   Dims d;
   float gamma, gam1, gam1_inv;
   const float* q;  // the state's FP32 copy
-  const double* area[10];
+  const double* met[10];
   const unsigned char* mask;
   unsigned stride;
   float bound;

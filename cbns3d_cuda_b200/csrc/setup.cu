@@ -96,8 +96,8 @@ __global__ void metrics_ghosts(Dims d, Met M) {
 // Node area vectors J*grad(xi), J*grad(eta), J*grad(zeta) and 1/J over the
 // ghosted box: the face normal of the reference is the mean of the two nodes'
 // J*grad(xi) (src/rec_riemann_kernel.cu:44-49), so it is formed once here.
-// The FP32 kernels use FP32 copies of the nine components (A32, may be
-// absent).
+// The FP32 kernels use FP32 copies of the nine components (A32; absent in FP64
+// contexts, where A has all ten, instead of the last four).
 struct Area32 {
   float* m[9];
 };
@@ -108,14 +108,13 @@ __global__ void area_kernel(Dims d, Met M, Met A, Area32 A32) {
   const int i = (int)(e % d.IG) - NG;
   const long r = e / d.IG;
   const long o = node_off(d, i, (int)(r % d.JG) - NG, (int)(r / d.JG) - NG);
-  const double J = M.m[9][o];
 #pragma unroll
-  for (int m = 0; m < 9; ++m) A.m[m][o] = M.m[m][o] * J;
-  A.m[9][o] = 1.0 / J;
-  if (A32.m[0]) {
-#pragma unroll
-    for (int m = 0; m < 9; ++m) A32.m[m][o] = (float)A.m[m][o];
+  for (int m = 0; m < 9; ++m) {
+    const double v = node_area(M.m, m, o);
+    if (A.m[m]) A.m[m][o] = v;
+    if (A32.m[m]) A32.m[m][o] = (float)v;
   }
+  A.m[9][o] = 1.0 / M.m[9][o];
 }
 
 struct Prims {

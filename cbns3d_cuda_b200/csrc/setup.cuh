@@ -6,8 +6,8 @@
 
 namespace cbns {
 
-// metrics, their ghost extension, and the node area vectors / 1/J (area32,
-// may be null: FP32 copies of the xi and eta area vectors).  wrap > 0 (O-grid):
+// metrics, their ghost extension, and the node area vectors / 1/J (those of area
+// and area32, FP32 copies, that are not null).  wrap > 0 (O-grid):
 // the nodes i < wrap and i >= IM - wrap take the metrics of the nodes
 // IM - 2*wrap away, before the ghost extension.
 cudaError_t launch_metrics(const Dims& d, const double* x, const double* y, const double* z, double* const met[10],

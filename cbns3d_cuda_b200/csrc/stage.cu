@@ -245,7 +245,7 @@ __device__ __forceinline__ void stage_body(const StageCore& a, const StageMaps* 
       tma::prefetch_4d(&tm->xi, xl, y0, z, 0);
       tma::prefetch_4d(&tm->eta, xc, y0 - 1, z, 3);
       tma::prefetch_4d(&tm->zeta, xc, y0, z + 1, 6);
-      tma::prefetch_4d(&tm->iJ, xc, y0, z, 9);
+      tma::prefetch_4d(&tm->iJ, xc, y0, z, 0);
       if (MODE >= 1 && !a.q0_is_src) tma::prefetch_4d(&tm->q0, xc, y0, z, 0);
       if (MODE >= 2 && !a.qp_is_src) tma::prefetch_4d(&tm->qp, xc, y0, z, 0);
     }
