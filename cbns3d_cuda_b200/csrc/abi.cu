@@ -244,7 +244,6 @@ StageArgs stage_args(cbns_ctx* c, const double* src, const double* q0, const dou
   a.q0 = q0;
   a.qp = qp;
   a.out = out;
-  fill_met(c, a.met);
   for (int m = 0; m < 10; ++m) a.area[m] = c->f.area[m];
   for (int m = 0; m < 4; ++m) a.dfv[m] = c->f.dfv[m];
   for (int m = 0; m < 6; ++m) a.prim[m] = c->f.prim[m];
@@ -254,7 +253,6 @@ StageArgs stage_args(cbns_ctx* c, const double* src, const double* q0, const dou
   a.ntile_i = c->ntile_i;
   a.ntile_j = c->ntile_j;
   a.kchunk = c->kchunk;
-  a.visdiv = c->ph.visdiv;
   a.sigma = sigma;
   a.lean = 0;
   a.mask = c->ph.precision == CBNS_PREC_HYBRID ? c->mask : nullptr;
@@ -1614,10 +1612,6 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
   }
   const int mode = c->ph.viscous ? 0 : 1;
   double* const P0 = c->qb[c->lq];
-  int done = 0;  // a finished run's stages return at once: off while they are timed
-  CK(cudaMemcpyAsync(&done, &c->st->done, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemsetAsync(&c->st->done, 0, sizeof(int), c->stream));
-  RET(sync(c));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   if (cudaEventCreate(&e1) != cudaSuccess) {
@@ -1625,6 +1619,10 @@ int cbns_autotune(cbns_ctx* c, int* chosen) {
     g_last = "cudaEventCreate failed";
     return CBNS_ERR_CUDA;
   }
+  int done = 0;  // a finished run's stages return at once: off while they are timed
+  CK(cudaMemcpyAsync(&done, &c->st->done, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemsetAsync(&c->st->done, 0, sizeof(int), c->stream));
+  RET(sync(c));
   // the faster of two rounds of three launches after one warm-up launch
   auto time_it = [&](int v, int kc, float* ms) -> int {
     c->stage_variant = v;

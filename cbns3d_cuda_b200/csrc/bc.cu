@@ -525,15 +525,15 @@ __device__ __forceinline__ void characteristic_state(const BCArgs& a, int dir, i
 // face node set earlier in the same call, so the state depends on the
 // buffer's interior only (not on its history).  Ghosts off those lines keep
 // their state.  Dims of at least 4 keep e off the other face.
-__global__ void bc_characteristic(const BCArgs a, int dir, int side0, int nsides) {
+__global__ void bc_characteristic(const BCArgs a, int dir) {
   if (a.check_done && a.st->done) return;
   const Dims& d = a.d;
   const int n0 = dir == 0 ? d.JM - 2 : d.IM;
   const int n1 = dir == 2 ? d.JM : d.KM - 2;
   const int nf = dir == 0 ? d.IM : dir == 1 ? d.JM : d.KM;
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= (long)nsides * n0 * n1) return;
-  const int side = side0 + (int)(t / ((long)n0 * n1));
+  if (t >= 2L * n0 * n1) return;
+  const int side = (int)(t / ((long)n0 * n1));
   const long r = t % ((long)n0 * n1);
   const int f0 = (int)(r % n0), f1 = (int)(r / n0);
   const int lb = side ? nf - 1 : 0;
@@ -683,9 +683,9 @@ cudaError_t launch_bc(const BCArgs& a, bool interior_prims, cudaStream_t s, int*
   }
   if (a.farfield) {
     if (a.characteristic) {
-      bc_characteristic<<<nblk(2L * (d.JM - 2) * (d.KM - 2), B), B, 0, s>>>(a, 0, 0, 2);
-      bc_characteristic<<<nblk(2L * d.IM * (d.KM - 2), B), B, 0, s>>>(a, 1, 0, 2);
-      bc_characteristic<<<nblk(2L * d.IM * d.JM, B), B, 0, s>>>(a, 2, 0, 2);
+      bc_characteristic<<<nblk(2L * (d.JM - 2) * (d.KM - 2), B), B, 0, s>>>(a, 0);
+      bc_characteristic<<<nblk(2L * d.IM * (d.KM - 2), B), B, 0, s>>>(a, 1);
+      bc_characteristic<<<nblk(2L * d.IM * d.JM, B), B, 0, s>>>(a, 2);
       nl += 3;
     }
     if (a.viscous || a.sigma) {

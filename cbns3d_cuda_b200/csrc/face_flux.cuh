@@ -49,8 +49,11 @@
 // flux carries ~1e-7 relative error anyway.  FP64 starts from the hardware's
 // 20-bit approximations and takes one third-order Householder iteration
 // (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
-// 1970), three and five fused operations, which leaves at most 1 ulp where the
-// library's correctly rounded forms cost several times as much.
+// 1970), three and five fused operations, which leaves at most 1 unit in the
+// last place (reciprocal) or 2 (roots) where the library's correctly rounded
+// forms cost several times as much; the flux is no further from 80-bit
+// arithmetic for it (above).  Values stored or compared outside the flux (the
+// primitives, the spectral radius) use the correctly rounded forms.
 // R is the arithmetic type (double for the plain path, float for the split path).
 #pragma once
 

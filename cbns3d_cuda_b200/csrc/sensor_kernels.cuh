@@ -62,8 +62,8 @@ struct MaskArgs {
 };
 
 // Widening of the decisions: a face takes WENO5 when the sensor chose WENO5
-// for a face of the same direction within SN_DILATE_ALONG faces along its own
-// grid line or SN_DILATE_ACROSS faces in the two other index directions.  A
+// for a face of the same direction within `along` faces along its own grid line
+// or `across` faces in the two other index directions.  A
 // discontinuity moves less than a cell per time step (CFL <= 1): along a line
 // it reaches at most one more node of the 6-node stencils near it, and a
 // curved front (a blast) reaches grid lines next to those it crossed at the
@@ -72,8 +72,8 @@ struct MaskArgs {
 // bits (pass 0), a pass along k that writes the decision bytes and counts and
 // lists the WENO5 faces (pass 1), each kind in its own list of
 // st->weno_listed[kind] entries that starts at the kind's first face index.
-// When the network runs only every n-th step, its
-// decisions must hold for n steps: widths 1 + n along and n across.
+// When the network runs only every n-th step, its decisions must hold for n
+// steps: widths 1 + n along and n across.
 struct DilateArgs {
   Dims d;
   const unsigned* in;      // decision bits

@@ -1,7 +1,8 @@
 // sensor_tc.cu - the sensor network's forward pass on the tcgen05 tensor
 // cores for a batch of feature vectors (BF16 operands, FP32 accumulation).
-// The same tile routine (tc_mlp.cuh) runs inside the hybrid stage kernel; this
-// kernel serves validation against the FP32 predictor and batch inference.
+// The same tile routine (tc_mlp.cuh) runs in the sweeps below, which decide the
+// faces of a hybrid block; the kernel on feature vectors serves validation
+// against the FP32 predictor and batch inference.
 #include "sensor_kernels.cuh"
 #include "tc_mlp.cuh"
 

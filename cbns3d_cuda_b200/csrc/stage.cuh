@@ -31,7 +31,6 @@ struct StageCore {
   double* out;         // stage output (5 fields), or the dense RHS array in mode 0
   float* out32;        // FP32 kernels: the FP32 copy of the stage output
   const float* src32;  // FP32 kernels: the FP32 copy of the stage input
-  const double* met[10];
   const double* area[10];  // J*grad(xi|eta|zeta) per node, then 1/J
   const double* dfv[4];    // viscous: the divergence of the node fluxes (visc.cu; FP32 elements in the FP32 kernels)
   double* prim[6];     // viscous: rho,u,v,w,p,T of the new interior state
@@ -41,7 +40,6 @@ struct StageCore {
   const float* area32[9];  // FP32 kernels: J*grad(xi), J*grad(eta), J*grad(zeta) per node in FP32
   int q0_is_src, qp_is_src;  // RK operands that equal the stage input (read from the ring)
   int ntile_i, ntile_j, kchunk;
-  int visdiv;          // CBNS_VISDIV_*
   int lean;            // viscous, stages 1 and 2 of a run: rho and p of the primitives are not read before stage 3
   int sigma;           // accumulate the interior spectral-radius max (inviscid stage 3)
 };

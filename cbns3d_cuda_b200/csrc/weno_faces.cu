@@ -114,7 +114,7 @@ __device__ __forceinline__ void weno_pair(const StageArgs& a, bool all, long w0,
 // pipe.  Built for 3 CTAs of 128 threads per SM (168 registers).  One launch of
 // a 256x256x128 hybrid step: 171 us with one face per thread from the FP64
 // state (256 threads, 80 registers), 149 us in pairs from its FP32 copy.
-__global__ void __launch_bounds__(WT, 3) weno_faces_kernel(const __grid_constant__ StageArgs a, int mode, long nf,
+__global__ void __launch_bounds__(WT, 3) weno_faces_kernel(const __grid_constant__ StageArgs a, int mode,
                                                            const int2* list) {
   __shared__ float2 stn[NEQ * 6][WT];
   const StepState* st = a.st;
@@ -158,7 +158,7 @@ cudaError_t weno_prepare() {
 cudaError_t launch_weno_faces(const StageArgs& a, int mode, long nfaces, const int2* list, cudaStream_t s) {
   cudaError_t e = weno_prepare();
   if (e != cudaSuccess || nfaces <= 0) return e;
-  weno_faces_kernel<<<g_weno_grid, WT, 0, s>>>(a, mode, nfaces, list);
+  weno_faces_kernel<<<g_weno_grid, WT, 0, s>>>(a, mode, list);
   return cudaGetLastError();
 }
 
