@@ -64,20 +64,20 @@ sys.path.insert(0, str(ROOT))
 # bytes per cell-update the kernel must move: per stage the stage input (40 B),
 # the metrics (80 B) and the output (40 B), plus the RK base in stages 2 and 3
 ALG_BYTES_PER_UPDATE = 560.0
-# FP64 FLOP the plain path executes per cell-update: dadd + dmul + 2 dfma
-# counted by ncu over a stage-2 launch of the plain stage kernel (4,660 per
-# node), times three stages
+# FP64 FLOP of the reference's arithmetic per cell-update: dadd + dmul + 2 dfma
+# counted by ncu over a stage-2 launch of the plain stage kernel in its first
+# form, which did the reference's operations one for one (4,660 per node), times
+# three stages
 FP64_FLOP_PER_UPDATE = 13980.0
 # nominal FP64 peak for context: 64 DFMA lanes per SM x 148 SMs x 2 FLOP x
 # 1.965 GHz; the fraction is taken against the DGEMM rate measured in the run
 FP64_NOMINAL_TFLOPS = 64 * 148 * 2 * 1.965e9 / 1e12
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per interior node
 # of one stage-2 launch of the stage kernel, from single ncu captures on the
-# shock-vortex case: plain FP64 kernel at 128x128x64, hybrid kernel at
-# 192x192x96 (inputs larger than L2 in both); traffic grows with the nodes of
-# a launch, so the figures scale to the bench grid
-FP64_STAGE_DRAM_BYTES_PER_NODE = 240.0
-HYBRID_STAGE_DRAM_BYTES_PER_NODE = 237.4
+# shock-vortex case at 192x192x96 (inputs larger than L2); traffic grows with the
+# nodes of a launch, so the figures scale to the bench grid
+FP64_STAGE_DRAM_BYTES_PER_NODE = 226.8
+HYBRID_STAGE_DRAM_BYTES_PER_NODE = 238.5
 
 
 def args():

@@ -88,8 +88,8 @@ struct GradSmem {
 // of 256 CTAs, so the tile is small, rows are read as float4 (broadcast), the
 // weight gradients take 2 x 2 outputs per thread (two 8-byte reads for four
 // products) and the last layer shares its sums among four threads a row.
-// 16,384 samples: 20.3 -> 14.2 us (128 tiles of 128 samples before; weights
-// loaded across their rows), 1.5 M samples 1050 -> 696 us; summing over clusters
+// 16,384 samples: 20.3 -> 12.8 us (128 tiles of 128 samples before; weights
+// loaded across their rows), 1.5 M samples 1050 -> 686 us; summing over clusters
 // of 4 or 8 CTAs first was slower (15.0 and 17.7 us, 1213 us).
 __global__ void __launch_bounds__(GT) mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
                                                       const unsigned char* __restrict__ Y, unsigned n, float pos_w,

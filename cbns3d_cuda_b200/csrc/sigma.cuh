@@ -3,7 +3,8 @@
 //
 // dt needs the largest FP64 spectral radius of the grid, and evaluating it at
 // every node (about 70 FP64 operations with four square roots) costs stage 3 a
-// tenth of its time.  Most nodes are far below the largest value already found,
+// tenth of its time in FP64 (1829 -> 1707 us on 256x256x128) and a fifth in the
+// hybrid (584 -> 458).  Most nodes are far below the largest value already found,
 // so a node is evaluated in FP64 only if its FP32 bound reaches it, or if its
 // squared sound speed is not safely positive in FP32 (the FP64 value may be a
 // NaN, which must end the run): the result is the same to the bit.

@@ -37,7 +37,10 @@
 // stages 1 / 2 / 3: hybrid 256x256x128 517 / 567 / 617 -> 385 / 446 / 584 (half
 // the instructions: 86 M warp instructions for 3.4 M nodes instead of 164 M);
 // split 193x161x129 464 / 480 / 519 -> 411 / 422 / 501; 64 viscous hybrid
-// blocks 1250 / 1418 / 1327 -> 954 / 1045 / 1009.
+// blocks 1250 / 1418 / 1327 -> 954 / 1045 / 1009.  Since then the bounded
+// spectral radius (sigma.cuh) took from stage 3 and the wider range of the FP32
+// weights (face_flux.cuh) added to the split: 387 / 440 / 469, 423 / 443 / 493
+// and 861 / 919 / 932.
 //
 // Hybrid (HYB): each face's sensor decision selects the linear upwind-5 flux,
 // evaluated here, or the characteristic WENO5 flux, evaluated before this

@@ -113,7 +113,8 @@ __device__ __forceinline__ void weno_pair(const StageArgs& a, bool all, long w0,
 // Bound by the stencil loads (24% of issue slots idle on them) and the FP32
 // pipe.  Built for 3 CTAs of 128 threads per SM (168 registers).  One launch of
 // a 256x256x128 hybrid step: 171 us with one face per thread from the FP64
-// state (256 threads, 80 registers), 149 us in pairs from its FP32 copy.
+// state (256 threads, 80 registers), 149 us in pairs from its FP32 copy (152
+// with a reciprocal per indicator, face_flux.cuh).
 __global__ void __launch_bounds__(WT, 3) weno_faces_kernel(const __grid_constant__ StageArgs a, int mode,
                                                            const int2* list) {
   __shared__ float2 stn[NEQ * 6][WT];

@@ -59,7 +59,9 @@ extern "C" {
 
 /* Arithmetic of the inviscid face flux. */
 #define CBNS_PREC_FP64    0  /* plain path, FP64 throughout (parity with the reference) */
-#define CBNS_PREC_SPLIT   1  /* FP32 reconstruction + flux, FP64 state/metrics/reductions */
+#define CBNS_PREC_SPLIT   1  /* FP32 reconstruction + flux, FP64 state/metrics/reductions;
+                              * the FP32 WENO5 weights hold characteristic differences
+                              * from node to node up to 1e10 */
 #define CBNS_PREC_HYBRID  2  /* SPLIT + learned shock sensor choosing WENO5 or upwind-5 */
 
 /* Where the viscous flux divergence is evaluated. */
